@@ -410,6 +410,14 @@ size_t fda_nms3d_workspace_bytes(int num_boxes);
 int fda_nms3d(const float *boxes_sorted, int num_boxes, float iou_threshold, void *workspace,
               size_t workspace_bytes, long long *keep, int *num_keep, void *stream);
 
+/* The same on unsorted boxes: ranks them by score on the device (stable, NaN first), then as above.  coordinate k of box i is
+ * boxes[i * box_stride + k * coord_stride], its score scores[i * score_stride]; keep[] holds indices of the input.  Up to
+ * 16384 boxes: fda_nms3d_scored_workspace_bytes is 0 beyond that (the ranking compares all pairs; sort instead). */
+size_t fda_nms3d_scored_workspace_bytes(int num_boxes);
+int fda_nms3d_scored(const float *boxes, long long box_stride, long long coord_stride, const float *scores,
+                     long long score_stride, int num_boxes, float iou_threshold, void *workspace, size_t workspace_bytes,
+                     long long *keep, int *num_keep, void *stream);
+
 /*
  * Backward pass that needs no workspace from the caller and allocates nothing: same inputs,
  * outputs and results as fda_backward, but the fp32 accumulation image sits in a fixed

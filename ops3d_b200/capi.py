@@ -21,7 +21,7 @@ EXPORTS = (
     "fda_peer_push_partials", "fda_peer_reduce_staged_cast", "fda_backward_bin_plan", "fda_backward_binned_part",
     "fda_pack_sampling", "fda_pack_sampling_backward", "fda_dcnv4_forward", "fda_dcnv4_backward",
     "fda_dcnv4_backward_workspace_bytes", "fda_dcnv4_output_size", "fda_roi_align3d_forward", "fda_roi_align3d_backward",
-    "fda_nms3d", "fda_nms3d_workspace_bytes", "fda_reload_config", "fda_group_reduce_cast", "fda_head_slice_cast_push",
+    "fda_nms3d", "fda_nms3d_workspace_bytes", "fda_nms3d_scored", "fda_nms3d_scored_workspace_bytes", "fda_reload_config", "fda_group_reduce_cast", "fda_head_slice_cast_push",
     "fda_backward_touched_rows", "fda_cast_grad_value_touched",
 )
 BWD_ZERO_IMAGE, BWD_RESUME, BWD_FINALIZE, BWD_BINNED_DONE, BWD_ZERO_TOUCHED = 1, 2, 4, 8, 16

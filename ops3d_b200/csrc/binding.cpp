@@ -246,18 +246,30 @@ at::Tensor nms_3d(const at::Tensor &dets, const at::Tensor &scores, const float 
     TORCH_CHECK(dets.dim() == 2 && dets.size(1) == 6, "boxes must be [N, 6] = (x1, y1, z1, x2, y2, z2)");
     TORCH_CHECK(scores.numel() == dets.size(0), "one score per box");
     const int n = (int)dets.size(0);
+    const auto narrow_type = [](at::ScalarType t) { return t == at::kFloat || t == at::kHalf || t == at::kBFloat16; };
+    at::Tensor keep = at::empty({n}, dets.options().dtype(at::kLong));
+    at::Tensor num = at::empty({1}, dets.options().dtype(at::kInt));
+    const auto stream = at::cuda::getCurrentCUDAStream().stream();
+    const size_t scored_bytes = fda_nms3d_scored_workspace_bytes(n);
+    if (scored_bytes > 0 && narrow_type(dets.scalar_type()) && narrow_type(scores.scalar_type())) {
+        // ranked on the device straight from the caller's (possibly strided) tensors
+        const at::Tensor boxes = dets.to(at::kFloat), flat = scores.reshape({-1}).to(at::kFloat);
+        at::Tensor workspace = at::empty({(int64_t)(scored_bytes / 8 + 1)}, dets.options().dtype(at::kLong));
+        raise_status(fda_nms3d_scored(boxes.data_ptr<float>(), boxes.stride(0), boxes.stride(1), flat.data_ptr<float>(), flat.stride(0),
+                                      n, threshold, workspace.data_ptr(), scored_bytes,
+                                      reinterpret_cast<long long *>(keep.data_ptr<int64_t>()), num.data_ptr<int>(), stream),
+                     "nms_3d");
+        return keep.narrow(0, 0, num.item<int>());  // the one host read: how many boxes survived
+    }
     // score order; the stable sort makes ties deterministic (earlier box first)
     at::Tensor order = std::get<1>(scores.reshape({-1}).sort(/*stable=*/true, /*dim=*/0, /*descending=*/true));
     at::Tensor sorted = dets.index_select(0, order).to(at::kFloat).contiguous();
     const size_t ws_bytes = fda_nms3d_workspace_bytes(n);
     at::Tensor workspace = at::empty({(int64_t)(ws_bytes / 8 + 1)}, dets.options().dtype(at::kLong));
-    at::Tensor keep = at::empty({n}, dets.options().dtype(at::kLong));
-    at::Tensor num = at::zeros({1}, dets.options().dtype(at::kInt));
     raise_status(fda_nms3d(sorted.data_ptr<float>(), n, threshold, workspace.data_ptr(), ws_bytes,
-                           reinterpret_cast<long long *>(keep.data_ptr<int64_t>()), num.data_ptr<int>(),
-                           at::cuda::getCurrentCUDAStream().stream()),
+                           reinterpret_cast<long long *>(keep.data_ptr<int64_t>()), num.data_ptr<int>(), stream),
                  "nms_3d");
-    const int64_t kept = num.item<int>();  // the one host read: how many boxes survived
+    const int64_t kept = num.item<int>();
     return order.index_select(0, keep.narrow(0, 0, kept));
 }
 

@@ -114,3 +114,20 @@ def test_roi_align3d_matches_reference_kernel_fixtures(name, z):
 def test_nms3d_matches_reference_kernel_fixtures(name, z):
     keep = _C.nms_3d(torch.from_numpy(z["boxes"]).cuda(), torch.from_numpy(z["scores"]).cuda(), float(z["threshold"]))
     assert keep.cpu().tolist() == z["keep"].tolist()
+
+
+@pytest.mark.parametrize("n", [64, 129, 4033, 4500])
+def test_nms3d_order_of_ties_and_far_columns(n):
+    """Scores with many ties, zeros of both signs, infinities and NaN (highest) from a strided tensor: the order of a stable
+    descending sort.  4033 boxes and more have columns with words beyond those a sweep thread holds in registers."""
+    gen = torch.Generator().manual_seed(n)
+    centre = torch.rand(n, 3, generator=gen) * 14
+    size = torch.rand(n, 3, generator=gen) * 12 + 2
+    scores = torch.randint(-20, 20, (n,), generator=gen).float() / 10
+    scores[:5] = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan")])
+    dets = torch.cat([centre - size / 2, centre + size / 2, scores[:, None]], 1).cuda()
+    order = torch.sort(dets[:, 6], stable=True, descending=True)[1]
+    boxes = dets[order, :6].cpu().numpy()
+    keep = ops3d.nms_nd(dets, 0.3)[0].cpu()
+    ranked = oracle.nms3d(boxes, -np.arange(n, dtype=np.float32), 0.3)   # already in score order
+    assert keep.tolist() == order.cpu()[ranked].tolist()

@@ -181,6 +181,324 @@ __global__ void __launch_bounds__(256) roi_align3d_backward_kernel(size_t total,
     }
 }
 
+// ---- separable form -------------------------------------------------------------------------------------
+// A sample's weights are products of one factor per axis, and so is its validity: the samples of a bin average to
+//   out[pd][ph][pw] = 1/count * sum_z Wz[pd][z] sum_y Wy[ph][y] sum_x Wx[pw][x] f[z][y][x]
+// with a small weight table per axis (nonzero on the bin's few voxels).  A block builds the tables of one ROI once for
+// its channels; a warp takes one channel and contracts axis after axis, plane by plane: about 10 x fewer operations than
+// eight corners per sample, and in the backward one reduction per voxel of the ROI and channel instead of eight per
+// sample (7x7x7 bins of 2x2x2 samples on a 9x17x21 ROI: 3.2 k against 22 k).  256 ROIs x 128 channels of a 16x32x64 volume:
+// forward 652 -> 152 us, backward 1723 -> 166 us.  What bounds it: shared-memory and L1 accesses of the short dot products.
+struct AxisTable {
+    float *w;     // [bins][size], zero outside [lo, hi]
+    int *lo, *hi; // [bins] first / last voxel of a bin (hi < lo: no valid sample)
+    int *b0, *b1; // [size] first / last bin that reads a voxel (b1 < b0: none)
+    int bins, size;
+};
+
+constexpr int kRoiThreads = 256;
+constexpr int kRoiChannels = 2;  // per warp at a time; 1 / 2 / 4: 484 / 317 / 399 us for the two passes below
+
+__host__ __device__ inline int roi_table_words(int bins, int size) { return bins * size + 2 * bins + 2 * size; }
+
+__device__ __forceinline__ AxisTable axis_table(float *mem, int bins, int size) {
+    AxisTable t;
+    t.w = mem;
+    t.lo = reinterpret_cast<int *>(mem + bins * size);
+    t.hi = t.lo + bins;
+    t.b0 = t.hi + bins;
+    t.b1 = t.b0 + size;
+    t.bins = bins;
+    t.size = size;
+    return t;
+}
+
+// One thread per bin; samples of a bin lie in increasing order.  The rows of t.w are zero.
+__device__ __forceinline__ void fill_axis_bin(const AxisTable &t, int p, float start, float bin, int grid, int order) {
+    int lo = 0, hi = -1;
+    for (int i = 0; i < grid; ++i) {
+        const float v = start + p * bin + ((float)i + .5f) * bin / (float)grid;
+        if (v < -1.0f || v > (float)t.size) continue;
+        int i0, i1;
+        float l, h;
+        axis_setup(v, t.size, i0, i1, l, h);
+        if (order == 0) {
+            l = l > 0.5f ? 1.f : 0.f;
+            h = 1.f - l;
+        }
+        if (hi < lo) lo = i0;
+        hi = i1;
+        t.w[p * t.size + i0] += h;
+        t.w[p * t.size + i1] += l;
+    }
+    t.lo[p] = lo;
+    t.hi[p] = hi;
+}
+
+struct RoiTables {
+    AxisTable z, y, x;
+    int z0, z1, y0, y1, x0, x1;  // voxel range of the ROI (every bin's range lies inside)
+};
+
+// Called by the whole block; ends with a barrier.
+template <typename RT>
+__device__ __forceinline__ RoiGeom build_roi_tables(RoiTables &t, float *mem, const RT *roi, float spatial_scale, int sampling_ratio,
+                                                    int order, int depth, int height, int width, int pd, int ph, int pw) {
+    const RoiGeom g = roi_geometry<RT>(roi, spatial_scale, sampling_ratio, pd, ph, pw);
+    t.x = axis_table(mem, pw, width);  // first: its rows are read as 16-byte vectors when the width is a multiple of four
+    t.y = axis_table(mem + roi_table_words(pw, width), ph, height);
+    t.z = axis_table(mem + roi_table_words(pw, width) + roi_table_words(ph, height), pd, depth);
+    const int tid = threadIdx.x, total = roi_table_words(pw, width) + roi_table_words(ph, height) + roi_table_words(pd, depth);
+    for (int i = tid; i < total; i += blockDim.x) mem[i] = 0.f;
+    __syncthreads();
+    for (int i = tid; i < pd + ph + pw; i += blockDim.x) {
+        if (i < pd) fill_axis_bin(t.z, i, g.start_d, g.bin_d, g.grid_d, order);
+        else if (i < pd + ph) fill_axis_bin(t.y, i - pd, g.start_h, g.bin_h, g.grid_h, order);
+        else fill_axis_bin(t.x, i - pd - ph, g.start_w, g.bin_w, g.grid_w, order);
+    }
+    __syncthreads();
+    for (int i = tid; i < depth + height + width; i += blockDim.x) {
+        const AxisTable &a = i < depth ? t.z : (i < depth + height ? t.y : t.x);
+        const int v = i < depth ? i : (i < depth + height ? i - depth : i - depth - height);
+        int first = 0, last = -1;
+        for (int p = 0; p < a.bins; ++p)
+            if (a.lo[p] <= v && v <= a.hi[p]) {
+                if (last < first) first = p;
+                last = p;
+            }
+        a.b0[v] = first;
+        a.b1[v] = last;
+    }
+    auto range = [](const AxisTable &a, int &v0, int &v1) {
+        v0 = a.size;
+        v1 = -1;
+        for (int p = 0; p < a.bins; ++p)
+            if (a.lo[p] <= a.hi[p]) {
+                v0 = min(v0, a.lo[p]);
+                v1 = max(v1, a.hi[p]);
+            }
+    };
+    range(t.z, t.z0, t.z1);
+    range(t.y, t.y0, t.y1);
+    range(t.x, t.x0, t.x1);
+    __syncthreads();
+    return g;
+}
+
+// Grid: (ROI, group of channels_per_block channels).  A warp takes kRoiChannels channels at a time (one weight and one set
+// of bin ranges then serve all of them, and their loads overlap).  Per warp and channel: [height][pw] rows contracted
+// along x, then the output tile [pd][ph][pw].  Lanes of both contractions: rows_per_step rows x pw bins, so that a lane
+// keeps its bin.
+template <typename T>
+__global__ void __launch_bounds__(kRoiThreads) roi_align3d_forward_separable_kernel(const T *__restrict__ features, const T *__restrict__ rois,
+                                                                                   float spatial_scale, int sampling_ratio, int order,
+                                                                                   int channels, int depth, int height, int width, int pd,
+                                                                                   int ph, int pw, int channels_per_block, T *__restrict__ out) {
+    constexpr int kC = kRoiChannels;
+    extern __shared__ __align__(16) float roi_smem[];
+    const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    RoiTables t;
+    const RoiGeom g = build_roi_tables<T>(t, roi_smem, rois + (size_t)n * 7, spatial_scale, sampling_ratio, order, depth, height, width, pd, ph, pw);
+    const int tables = roi_table_words(pd, depth) + roi_table_words(ph, height) + roi_table_words(pw, width);
+    const int bins = pd * ph * pw, rows_size = height * pw;
+    float *rows = roi_smem + ((tables + 3) & ~3) + warp * kC * (rows_size + bins), *tile = rows + kC * rows_size;
+    const int rows_per_step = 32 / pw, lane_row = lane / pw, p = lane - lane_row * pw;
+    const bool used = lane_row < rows_per_step;
+    const int xlo = used ? t.x.lo[p] : 0, xhi = used ? t.x.hi[p] : -1;
+    const float *wx = t.x.w + (used ? p : 0) * width;
+    const int c_end = min(channels, ((int)blockIdx.y + 1) * channels_per_block);
+    const size_t volume = (size_t)depth * height * width;
+    for (int c = blockIdx.y * channels_per_block + warp * kC; c < c_end; c += warps * kC) {
+        const T *vol = features + ((size_t)g.batch * channels + c) * volume;
+        size_t of[kC];  // a channel beyond the last one repeats the last one; its result is dropped
+#pragma unroll
+        for (int k = 0; k < kC; ++k) of[k] = (size_t)min(k, c_end - 1 - c) * volume;
+        for (int i = lane; i < kC * bins; i += 32) tile[i] = 0.f;
+        for (int z = t.z0; z <= t.z1; ++z) {
+            if (used)
+                for (int y = t.y0 + lane_row; y <= t.y1; y += rows_per_step) {
+                    const T *src = vol + ((size_t)z * height + y) * width;
+                    float acc[kC];
+#pragma unroll
+                    for (int k = 0; k < kC; ++k) acc[k] = 0.f;
+#pragma unroll 2
+                    for (int x = xlo; x <= xhi; ++x) {
+                        const float w = wx[x];
+#pragma unroll
+                        for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, ldf<T>(src + of[k] + x), acc[k]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < kC; ++k) rows[k * rows_size + y * pw + p] = acc[k];
+                }
+            __syncwarp();
+            if (used)
+                for (int q = lane_row; q < ph; q += rows_per_step) {
+                    const float *wy = t.y.w + q * height;
+                    float acc[kC];
+#pragma unroll
+                    for (int k = 0; k < kC; ++k) acc[k] = 0.f;
+#pragma unroll 2
+                    for (int y = t.y.lo[q]; y <= t.y.hi[q]; ++y) {
+                        const float w = wy[y];
+#pragma unroll
+                        for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, rows[k * rows_size + y * pw + p], acc[k]);
+                    }
+                    for (int d = t.z.b0[z]; d <= t.z.b1[z]; ++d) {
+                        const float w = t.z.w[d * depth + z];
+                        float *o = tile + (d * ph + q) * pw + p;
+#pragma unroll
+                        for (int k = 0; k < kC; ++k) o[k * bins] = fmaf(w, acc[k], o[k * bins]);
+                    }
+                }
+            __syncwarp();
+        }
+        T *dst = out + ((size_t)n * channels + c) * (size_t)bins;
+        const int valid = min(kC, c_end - c) * bins;
+        for (int i = lane; i < valid; i += 32) dst[i] = cvt_out<T>(tile[i] / g.count);
+        __syncwarp();
+    }
+}
+
+// The transpose, plane by plane: grad rows contracted along z, expanded along y, then along x into the voxels of the ROI's
+// plane, which are added to grad_features: kVec = 4 consecutive voxels per 16-byte reduction where the rows allow it.
+template <typename T, int kVec>
+__global__ void __launch_bounds__(kRoiThreads) roi_align3d_backward_separable_kernel(const T *__restrict__ grad_out, const float *__restrict__ rois,
+                                                                                    float spatial_scale, int sampling_ratio, int order,
+                                                                                    int channels, int depth, int height, int width, int pd,
+                                                                                    int ph, int pw, int channels_per_block,
+                                                                                    float *__restrict__ grad_features) {
+    constexpr int kC = kRoiChannels;
+    extern __shared__ __align__(16) float roi_smem[];
+    const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    RoiTables t;
+    const RoiGeom g = build_roi_tables<float>(t, roi_smem, rois + (size_t)n * 7, spatial_scale, sampling_ratio, order, depth, height, width, pd, ph, pw);
+    const int tables = roi_table_words(pd, depth) + roi_table_words(ph, height) + roi_table_words(pw, width);
+    const int bins = pd * ph * pw, rows_size = height * pw, plane_size = ph * pw;
+    float *rows = roi_smem + ((tables + 3) & ~3) + warp * kC * (rows_size + bins + plane_size), *tile = rows + kC * rows_size,
+          *plane = tile + kC * bins;
+    const int rows_per_step = 32 / pw, lane_row = lane / pw, p = lane - lane_row * pw;
+    const bool used = lane_row < rows_per_step;
+    const int ny = t.y1 - t.y0 + 1, v0 = t.x0 / kVec, nv = t.x1 / kVec - v0 + 1;  // vectors per row of the ROI
+    const int c_end = min(channels, ((int)blockIdx.y + 1) * channels_per_block);
+    const size_t volume = (size_t)depth * height * width;
+    if (t.z1 < t.z0 || ny <= 0 || t.x1 < t.x0) return;  // no valid sample (uniform over the block)
+    for (int c = blockIdx.y * channels_per_block + warp * kC; c < c_end; c += warps * kC) {
+        float *vol = grad_features + ((size_t)g.batch * channels + c) * volume;
+        const T *src = grad_out + ((size_t)n * channels + c) * (size_t)bins;
+        const int valid = min(kC, c_end - c);
+        for (int i = lane; i < kC * bins; i += 32) tile[i] = i < valid * bins ? ldf<T>(src + i) / g.count : 0.f;
+        __syncwarp();
+        for (int z = t.z0; z <= t.z1; ++z) {
+            for (int i = lane; i < plane_size; i += 32) {
+                float acc[kC];
+#pragma unroll
+                for (int k = 0; k < kC; ++k) acc[k] = 0.f;
+                for (int d = t.z.b0[z]; d <= t.z.b1[z]; ++d) {
+                    const float w = t.z.w[d * depth + z];
+#pragma unroll
+                    for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, tile[k * bins + d * plane_size + i], acc[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < kC; ++k) plane[k * plane_size + i] = acc[k];
+            }
+            __syncwarp();
+            if (used)
+                for (int y = t.y0 + lane_row; y <= t.y1; y += rows_per_step) {
+                    float acc[kC];
+#pragma unroll
+                    for (int k = 0; k < kC; ++k) acc[k] = 0.f;
+                    for (int q = t.y.b0[y]; q <= t.y.b1[y]; ++q) {
+                        const float w = t.y.w[q * height + y];
+#pragma unroll
+                        for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, plane[k * plane_size + q * pw + p], acc[k]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < kC; ++k) rows[k * rows_size + y * pw + p] = acc[k];
+                }
+            __syncwarp();
+            int r = lane / nv, v = lane - r * nv;            // row and vector of this lane, advanced without divisions
+            const int step_r = 32 / nv, step_v = 32 - step_r * nv;
+            while (r < ny) {
+                const int y = t.y0 + r, x = (v0 + v) * kVec;
+                float acc[kC][kVec];
+#pragma unroll
+                for (int k = 0; k < kC; ++k)
+#pragma unroll
+                    for (int e = 0; e < kVec; ++e) acc[k][e] = 0.f;
+                int first = t.x.bins, last = -1;
+#pragma unroll
+                for (int e = 0; e < kVec; ++e)
+                    if (t.x.b0[x + e] <= t.x.b1[x + e]) {
+                        first = min(first, t.x.b0[x + e]);
+                        last = max(last, t.x.b1[x + e]);
+                    }
+                for (int b = first; b <= last; ++b) {
+                    const float *w = t.x.w + b * width + x;
+                    float we[kVec];
+                    if constexpr (kVec == 4) {
+                        const float4 w4 = *reinterpret_cast<const float4 *>(w);
+                        we[0] = w4.x; we[1] = w4.y; we[2] = w4.z; we[3] = w4.w;
+                    } else {
+                        we[0] = w[0];
+                    }
+#pragma unroll
+                    for (int k = 0; k < kC; ++k) {
+                        const float u = rows[k * rows_size + y * pw + b];
+#pragma unroll
+                        for (int e = 0; e < kVec; ++e) acc[k][e] = fmaf(we[e], u, acc[k][e]);
+                    }
+                }
+                float *dst = vol + ((size_t)z * height + y) * width + x;
+#pragma unroll
+                for (int k = 0; k < kC; ++k)
+                    if (k < valid) {
+                        if constexpr (kVec == 4)
+                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + k * volume), "f"(acc[k][0]),
+                                         "f"(acc[k][1]), "f"(acc[k][2]), "f"(acc[k][3]) : "memory");
+                        else
+                            atomicAdd(dst + k * volume, acc[k][0]);
+                    }
+                r += step_r;
+                v += step_v;
+                if (v >= nv) {
+                    v -= nv;
+                    ++r;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// Launch shape of the separable kernels, or false: a row of bins wider than a warp, or tables and tiles beyond shared
+// memory even for one warp, take the element-wise kernels.
+struct RoiLaunch {
+    int threads, channels_per_block;
+    size_t smem;
+    dim3 grid;
+};
+bool roi_launch(int num_rois, int channels, int depth, int height, int width, int pd, int ph, int pw, bool backward, RoiLaunch &l) {
+    if (pw > 32 || (double)pd * depth + (double)ph * height + (double)pw * width > 40000.0 || (double)pd * ph * pw > 40000.0) return false;
+    const size_t tables = (size_t)roi_table_words(pd, depth) + roi_table_words(ph, height) + roi_table_words(pw, width);
+    const size_t per_warp = kRoiChannels * ((size_t)height * pw + (size_t)pd * ph * pw + (backward ? (size_t)ph * pw : 0));
+    l.threads = kRoiThreads;
+    auto bytes = [&]() { return (((tables + 3) & ~(size_t)3) + (size_t)(l.threads / 32) * per_warp) * sizeof(float); };
+    while (l.threads > 32 && bytes() > 56 * 1024) l.threads /= 2;  // four blocks of an SM
+    l.smem = bytes();
+    if (l.smem > 200 * 1024) return false;
+    // the tables are shared by a block's channels: up to 64 of them while the SMs still get six blocks each
+    l.channels_per_block = l.threads / 32 * kRoiChannels;
+    while (l.channels_per_block < 64 && (size_t)num_rois * ((channels + 2 * l.channels_per_block - 1) / (2 * l.channels_per_block)) >= 148 * 6)
+        l.channels_per_block *= 2;
+    l.grid = dim3((unsigned)num_rois, (unsigned)((channels + l.channels_per_block - 1) / l.channels_per_block));
+    return l.grid.y <= 65535;
+}
+
+template <typename K>
+cudaError_t roi_opt_in(K kernel, size_t smem) {
+    return smem > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) : cudaSuccess;
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // NMS 3D
 // ---------------------------------------------------------------------------------------------------------
@@ -435,6 +753,21 @@ extern "C" int fda_roi_align3d_forward(const void *features, const void *rois, v
     const size_t total = (size_t)num_rois * channels * pooled_depth * pooled_height * pooled_width;
     if (total == 0) return FDA_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    RoiLaunch l;
+    if (roi_launch(num_rois, channels, depth, height, width, pooled_depth, pooled_height, pooled_width, false, l)) {
+        auto launch = [&](auto kernel, auto *typed) -> int {
+            using T = std::remove_pointer_t<decltype(typed)>;
+            const cudaError_t e = roi_opt_in(kernel, l.smem);
+            if (e != cudaSuccess) return status_of(e);
+            kernel<<<l.grid, l.threads, l.smem, st>>>(static_cast<const T *>(features), static_cast<const T *>(rois), spatial_scale,
+                                                      sampling_ratio, order, channels, depth, height, width, pooled_depth, pooled_height,
+                                                      pooled_width, l.channels_per_block, typed);
+            return status_of(cudaGetLastError());
+        };
+        if (dtype == FDA_DTYPE_F32) return launch(roi_align3d_forward_separable_kernel<float>, static_cast<float *>(output));
+        if (dtype == FDA_DTYPE_F16) return launch(roi_align3d_forward_separable_kernel<__half>, static_cast<__half *>(output));
+        return launch(roi_align3d_forward_separable_kernel<__nv_bfloat16>, static_cast<__nv_bfloat16 *>(output));
+    }
     const unsigned g = grid_for(total);
 #define FDA_ROI_FWD(T)                                                                                                     \
     roi_align3d_forward_kernel<T><<<g, 256, 0, st>>>(total, static_cast<const T *>(features), static_cast<const T *>(rois),    \
@@ -459,6 +792,24 @@ extern "C" int fda_roi_align3d_backward(const void *grad_output, const float *ro
     const size_t total = (size_t)num_rois * channels * pooled_depth * pooled_height * pooled_width;
     if (total == 0) return FDA_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    RoiLaunch l;
+    if (roi_launch(num_rois, channels, depth, height, width, pooled_depth, pooled_height, pooled_width, true, l)) {
+        const bool vec = width % 4 == 0 && (reinterpret_cast<uintptr_t>(grad_features) & 15u) == 0;
+        auto launch = [&](auto kernel, const auto *typed) -> int {
+            const cudaError_t e = roi_opt_in(kernel, l.smem);
+            if (e != cudaSuccess) return status_of(e);
+            kernel<<<l.grid, l.threads, l.smem, st>>>(typed, rois, spatial_scale, sampling_ratio, order, channels, depth, height, width,
+                                                      pooled_depth, pooled_height, pooled_width, l.channels_per_block, grad_features);
+            return status_of(cudaGetLastError());
+        };
+        auto typed_launch = [&](const auto *typed) -> int {
+            using T = std::remove_cv_t<std::remove_pointer_t<decltype(typed)>>;
+            return vec ? launch(roi_align3d_backward_separable_kernel<T, 4>, typed) : launch(roi_align3d_backward_separable_kernel<T, 1>, typed);
+        };
+        if (grad_output_dtype == FDA_DTYPE_F32) return typed_launch(static_cast<const float *>(grad_output));
+        if (grad_output_dtype == FDA_DTYPE_F16) return typed_launch(static_cast<const __half *>(grad_output));
+        return typed_launch(static_cast<const __nv_bfloat16 *>(grad_output));
+    }
     const unsigned g = grid_for(total);
 #define FDA_ROI_BWD(T)                                                                                                      \
     roi_align3d_backward_kernel<T><<<g, 256, 0, st>>>(total, static_cast<const T *>(grad_output), rois, spatial_scale,           \

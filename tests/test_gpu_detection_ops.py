@@ -131,3 +131,21 @@ def test_nms3d_order_of_ties_and_far_columns(n):
     keep = ops3d.nms_nd(dets, 0.3)[0].cpu()
     ranked = oracle.nms3d(boxes, -np.arange(n, dtype=np.float32), 0.3)   # already in score order
     assert keep.tolist() == order.cpu()[ranked].tolist()
+
+
+@pytest.mark.parametrize("size", [(1, 1, 1), (2, 5, 7), (3, 2, 31), (2, 1, 33)])   # rows of bins: one, 4 of a warp, one lane idle, too wide
+@pytest.mark.parametrize("width", [8, 9, 40])                                      # 16-byte reductions or not; more than 32 vectors
+def test_roi_align3d_row_shapes(size, width):
+    N, C, D, H = 2, 9, 5, 6
+    gen = torch.Generator().manual_seed(width)
+    feats = torch.randn(N, C, D, H, width * (4 if width == 40 else 1), generator=gen)
+    rois = torch.cat([_rois(3, N, D, H, feats.shape[4], seed=width), torch.tensor([[0, -40.0, -40, -40, -30, -30, -30], [1, 0, 0, 0, 300, 5, 4]])])
+    f = feats.cuda().requires_grad_(True)
+    for ratio in (2, 0):
+        out = ops3d.roi_align_3d(f, rois.cuda(), size, 1.0, ratio, 1)
+        gout = torch.randn(out.shape, generator=gen)
+        (grad,) = torch.autograd.grad(out, f, gout.cuda())
+        want = oracle.roi_align3d_forward(feats.numpy(), rois.numpy(), size, 1.0, ratio, 1)
+        want_g = oracle.roi_align3d_backward(gout.numpy(), rois.numpy(), tuple(feats.shape), 1.0, ratio, 1)
+        assert np.abs(out.detach().cpu().numpy() - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
+        assert np.abs(grad.cpu().numpy() - want_g).max() <= 1e-4 * max(1.0, np.abs(want_g).max())

@@ -5,7 +5,6 @@ features ``[N, C, D, H, W]``; rois ``[n, 7]`` = (batch index, x1, y1, z1, x2, y2
 ``[n, C, out_d, out_h, out_w]``.  Gradients flow to ``features`` only (as in the reference); they are accumulated in
 fp32 and returned in the dtype of ``features``.
 """
-import torch
 import torch.nn as nn
 from torch.autograd import Function
 
@@ -20,7 +19,7 @@ def _require():
 
 class RoIAlign3DFunction(Function):
     @staticmethod
-    def forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio=0, order=1):
+    def apply(features, rois, output_size, spatial_scale, sampling_ratio=0, order=1):
         if isinstance(output_size, int):
             out_d = out_h = out_w = output_size
         elif isinstance(output_size, tuple):
@@ -28,25 +27,7 @@ class RoIAlign3DFunction(Function):
             out_d, out_h, out_w = output_size
         else:
             raise TypeError('"output_size" must be an integer or tuple of integers')
-        ctx.spatial_scale, ctx.sampling_ratio, ctx.order = spatial_scale, sampling_ratio, order
-        ctx.save_for_backward(rois)
-        ctx.feature_size, ctx.feature_dtype = features.size(), features.dtype
-        output = features.new_empty(rois.size(0), features.size(1), out_d, out_h, out_w)
-        _require().roi_align_3d_forward(features.contiguous(), rois.to(features.dtype).contiguous(), output, out_d, out_h, out_w,
-                                        spatial_scale, sampling_ratio, order)
-        return output
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        (rois,) = ctx.saved_tensors
-        grad_input = None
-        if ctx.needs_input_grad[0]:
-            out_d, out_h, out_w = grad_output.shape[2:]
-            accum = torch.zeros(ctx.feature_size, dtype=torch.float32, device=grad_output.device)
-            _require().roi_align_3d_backward(grad_output.contiguous(), rois.float().contiguous(), accum, out_d, out_h, out_w,
-                                             ctx.spatial_scale, ctx.sampling_ratio, ctx.order)
-            grad_input = accum.to(ctx.feature_dtype)
-        return grad_input, None, None, None, None, None
+        return _require().roi_align_3d(features, rois, out_d, out_h, out_w, spatial_scale, sampling_ratio, order)
 
 
 roi_align_3d = RoIAlign3DFunction.apply

@@ -76,7 +76,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 def build_binding(force: bool = False, verbose: bool = False) -> str:
     src = os.path.join(CSRC, "binding.cpp")
-    if not force and _newer(EXT, [src, os.path.join(ROOT, "include", "fda_b200.h"), LIB]):
+    if not force and _newer(EXT, [src, os.path.join(CSRC, "autograd_nodes.h"), os.path.join(ROOT, "include", "fda_b200.h"), LIB]):
         return EXT
     import torch
     from torch.utils import cpp_extension as ce

@@ -9,11 +9,13 @@
 // with the argument meaning and error behaviour of csrc/flash_deform_attn.h:7-52 and
 // csrc/cuda/flash_deform_attn_cuda.cu:20-179: RuntimeError for CPU / non-contiguous tensors and
 // for batch % min(batch, im2col_step) != 0, ValueError for an unsupported level or point count.
+// flash_deform_attn, dcnv4 and roi_align_3d are their differentiable forms (autograd_nodes.h), what the Python Functions call.
 // This file only checks tensors, allocates outputs from torch's allocator, and forwards raw
 // pointers plus the current CUDA stream; all arithmetic lives behind the C ABI.
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include <stdexcept>
@@ -21,8 +23,15 @@
 #include <vector>
 
 #include "../../include/fda_b200.h"
+#include "autograd_nodes.h"
 
 namespace {
+
+// Uninitialised CUDA memory straight from the allocator (no dispatcher round: 1 us less per tensor).
+at::Tensor empty_on(const at::Tensor &like, at::IntArrayRef size, at::ScalarType dtype) {
+    return at::detail::empty_cuda(size, dtype, like.device(), std::nullopt);
+}
+at::Tensor empty_as(const at::Tensor &like) { return empty_on(like, like.sizes(), like.scalar_type()); }
 
 int dtype_code(const at::Tensor &t, const char *name) {
     switch (t.scalar_type()) {
@@ -86,7 +95,7 @@ at::Tensor flash_deform_attn_forward(const at::Tensor &value, const at::Tensor &
     const int vdt = dtype_code(value, "value"), pdt = dtype_code(sampling_loc_attn, "sampling_loc_attn");
     c10::cuda::CUDAGuard guard(value.device());
     if (d.Q == 0 || d.B == 0) return at::zeros({d.B, d.Q, d.G * d.D}, value.options());
-    at::Tensor output = at::empty({d.B, d.Q, d.G * d.D}, value.options());
+    at::Tensor output = empty_on(value, {d.B, d.Q, d.G * d.D}, value.scalar_type());
     const int rc = fda_forward(value.data_ptr(), spatial_shapes.data_ptr<int64_t>(), level_start_index.data_ptr<int64_t>(),
                                sampling_loc_attn.data_ptr(), output.data_ptr(), d.B, d.N, d.G, d.D, d.L, d.Q, K, vdt, pdt,
                                im2col_step, d_stride, block_thread, use_reg ? 1 : 0,
@@ -107,13 +116,13 @@ std::vector<at::Tensor> flash_deform_attn_backward(const at::Tensor &value, cons
     const int vdt = dtype_code(value, "value"), pdt = dtype_code(sampling_loc_attn, "sampling_loc_attn");
     c10::cuda::CUDAGuard guard(value.device());
     if (d.Q == 0 || d.B == 0) return {at::zeros_like(value), at::zeros_like(sampling_loc_attn)};
-    at::Tensor grad_value = at::empty_like(value);
-    at::Tensor grad_packed = at::empty_like(sampling_loc_attn);
+    at::Tensor grad_value = empty_as(value);
+    at::Tensor grad_packed = empty_as(sampling_loc_attn);
     const size_t ws_bytes = fda_backward_workspace_bytes(d.B, d.N, d.G, d.D, d.L, d.Q, K, vdt, pdt);
     at::Tensor workspace;
     void *ws_ptr = nullptr;
     if (ws_bytes > 0) {
-        workspace = at::empty({(int64_t)((ws_bytes + 3) / sizeof(float))}, value.options().dtype(at::kFloat));
+        workspace = empty_on(value, {(int64_t)((ws_bytes + 3) / sizeof(float))}, at::kFloat);
         ws_ptr = workspace.data_ptr();
     }
     const int rc = fda_backward(value.data_ptr(), spatial_shapes.data_ptr<int64_t>(), level_start_index.data_ptr<int64_t>(),
@@ -122,6 +131,41 @@ std::vector<at::Tensor> flash_deform_attn_backward(const at::Tensor &value, cons
                                 im2col_step, d_stride, block_thread, at::cuda::getCurrentCUDAStream().stream());
     raise_status(rc, "flash_deform_attn_backward");
     return {grad_value, grad_packed};
+}
+
+// FlashDeformAttnFunction.apply: the forward, and the node of its backward when a gradient is wanted.
+struct FlashDeformAttnBackward : public fda_nodes::SavedNode {
+    int im2col_step, K;
+    std::string name() const override { return "FlashDeformAttnFunctionBackward"; }
+    torch::autograd::variable_list apply(torch::autograd::variable_list &&grads) override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (!grads[0].defined()) return {at::Tensor(), at::Tensor()};
+        const bool recording = at::GradMode::is_enabled() && grads[0].requires_grad();
+        at::NoGradGuard no_grad;
+        auto r = flash_deform_attn_backward(unpack(0), unpack(1), unpack(2), unpack(3), grads[0].contiguous(), im2col_step, K, 1, 0);
+        return fda_nodes::once_differentiable({r[0], r[1]}, recording);
+    }
+};
+
+at::Tensor flash_deform_attn(const at::Tensor &value, const at::Tensor &spatial_shapes, const at::Tensor &level_start_index,
+                             const at::Tensor &sampling_loc_attn, int im2col_step, int K, bool use_reg) {
+    const int64_t L = spatial_shapes.size(0), last = sampling_loc_attn.size(-1);
+    if (last != L * K * 4)
+        throw std::invalid_argument("sampling_loc_attn last dimension (" + std::to_string(last) +
+                                    ") does not match value_spatial_shapes level count L=" + std::to_string(L) + " and K=" +
+                                    std::to_string(K) + " (expected " + std::to_string(L * K * 4) + ")");
+    at::Tensor output = flash_deform_attn_forward(value, spatial_shapes, level_start_index, sampling_loc_attn, im2col_step, K, 8, 0, use_reg);
+    if (fda_nodes::needs_node({value, sampling_loc_attn})) {
+        auto node = std::make_shared<FlashDeformAttnBackward>();
+        node->im2col_step = im2col_step;
+        node->K = K;
+        node->save(0, value);
+        node->save(1, spatial_shapes);
+        node->save(2, level_start_index);
+        node->save(3, sampling_loc_attn);
+        fda_nodes::connect(node, output, torch::autograd::collect_next_edges(value, sampling_loc_attn));
+    }
+    return output;
 }
 
 // DCNv4-3D with the positional signatures of the reference's binding (csrc/dcnv4.h:7-61, registered at
@@ -159,7 +203,7 @@ at::Tensor dcnv4_forward(const at::Tensor &value, const at::Tensor &p_offset, co
     TORCH_CHECK(p_offset.size(0) == d.B && p_offset.size(1) == Do && p_offset.size(2) == Ho && p_offset.size(3) == Wo,
                 "p_offset spatial shape does not match the output volume");
     c10::cuda::CUDAGuard guard(value.device());
-    at::Tensor output = at::empty({d.B, Do, Ho, Wo, d.C}, value.options());
+    at::Tensor output = empty_on(value, {d.B, Do, Ho, Wo, d.C}, value.scalar_type());
     raise_status(fda_dcnv4_forward(value.data_ptr(), p_offset.data_ptr(), output.data_ptr(), d.B, d.Din, d.Hin, d.Win, group,
                                    group_channels, kernel, stride, pad, dilation, offset_scale, remove_center, softmax ? 1 : 0,
                                    d.padded, dtype_code(value, "value"), im2col_step,
@@ -183,13 +227,13 @@ std::vector<at::Tensor> dcnv4_backward(const at::Tensor &value, const at::Tensor
     const int pad[3] = {pad_d, pad_h, pad_w}, dilation[3] = {dilation_d, dilation_h, dilation_w};
     const int vdt = dtype_code(value, "value");
     c10::cuda::CUDAGuard guard(value.device());
-    at::Tensor grad_value = at::empty_like(value);
-    at::Tensor grad_offset = at::empty_like(p_offset);
+    at::Tensor grad_value = empty_as(value);
+    at::Tensor grad_offset = empty_as(p_offset);
     const size_t ws_bytes = fda_dcnv4_backward_workspace_bytes(d.B, d.Din, d.Hin, d.Win, group, group_channels, vdt);
     at::Tensor workspace;
     void *ws_ptr = nullptr;
     if (ws_bytes > 0) {
-        workspace = at::empty({(int64_t)((ws_bytes + 3) / sizeof(float))}, value.options().dtype(at::kFloat));
+        workspace = empty_on(value, {(int64_t)((ws_bytes + 3) / sizeof(float))}, at::kFloat);
         ws_ptr = workspace.data_ptr();
     }
     raise_status(fda_dcnv4_backward(value.data_ptr(), p_offset.data_ptr(), grad_output.data_ptr(), grad_value.data_ptr(),
@@ -198,6 +242,44 @@ std::vector<at::Tensor> dcnv4_backward(const at::Tensor &value, const at::Tensor
                                     im2col_step, at::cuda::getCurrentCUDAStream().stream()),
                  "dcnv4_backward");
     return {grad_value, grad_offset};
+}
+
+// DCNv4Function.apply.
+struct DCNv4Args {
+    std::array<int, 3> kernel, stride, pad, dilation;
+    int group, group_channels, im2col_step, remove_center;
+    float offset_scale;
+    bool softmax;
+};
+struct DCNv4Backward : public fda_nodes::SavedNode {
+    DCNv4Args a;
+    std::string name() const override { return "DCNv4FunctionBackward"; }
+    torch::autograd::variable_list apply(torch::autograd::variable_list &&grads) override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (!grads[0].defined()) return {at::Tensor(), at::Tensor()};
+        const bool recording = at::GradMode::is_enabled() && grads[0].requires_grad();
+        at::NoGradGuard no_grad;
+        auto r = dcnv4_backward(unpack(0), unpack(1), a.kernel[0], a.kernel[1], a.kernel[2], a.stride[0], a.stride[1], a.stride[2],
+                                a.pad[0], a.pad[1], a.pad[2], a.dilation[0], a.dilation[1], a.dilation[2], a.group, a.group_channels,
+                                a.offset_scale, a.im2col_step, grads[0].contiguous(), a.remove_center, 8, 0, a.softmax);
+        return fda_nodes::once_differentiable({r[0], r[1]}, recording);
+    }
+};
+
+at::Tensor dcnv4(const at::Tensor &value, const at::Tensor &p_offset, std::array<int, 3> kernel, std::array<int, 3> stride,
+                 std::array<int, 3> pad, std::array<int, 3> dilation, int group, int group_channels, float offset_scale,
+                 int im2col_step, int remove_center, bool softmax) {
+    at::Tensor output = dcnv4_forward(value, p_offset, kernel[0], kernel[1], kernel[2], stride[0], stride[1], stride[2], pad[0], pad[1],
+                                      pad[2], dilation[0], dilation[1], dilation[2], group, group_channels, offset_scale, im2col_step,
+                                      remove_center, 8, 0, softmax);
+    if (fda_nodes::needs_node({value, p_offset})) {
+        auto node = std::make_shared<DCNv4Backward>();
+        node->a = {kernel, stride, pad, dilation, group, group_channels, im2col_step, remove_center, offset_scale, softmax};
+        node->save(0, value);
+        node->save(1, p_offset);
+        fda_nodes::connect(node, output, torch::autograd::collect_next_edges(value, p_offset));
+    }
+    return output;
 }
 
 // ROI-Align 3D and NMS 3D with the reference's binding signatures (csrc/roi_align_3d.h:96-136, csrc/nms_3d.h:28-44):
@@ -237,6 +319,49 @@ void roi_align_3d_backward(at::Tensor top_grad, at::Tensor rois, at::Tensor bott
                                           sampling_ratio, order, dtype_code(top_grad, "top_grad"),
                                           at::cuda::getCurrentCUDAStream().stream()),
                  "roi_align_3d_backward");
+}
+
+// RoIAlign3DFunction.apply: the gradient is accumulated in fp32 and returned in the dtype of the features.
+struct RoIAlign3DBackward : public fda_nodes::SavedNode {
+    std::vector<int64_t> feature_size;
+    at::ScalarType feature_dtype;
+    float spatial_scale;
+    int sampling_ratio, order;
+    std::string name() const override { return "RoIAlign3DFunctionBackward"; }
+    torch::autograd::variable_list apply(torch::autograd::variable_list &&grads) override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (!grads[0].defined()) return {at::Tensor()};
+        at::NoGradGuard no_grad;
+        const at::Tensor &g = grads[0];
+        c10::cuda::CUDAGuard guard(g.device());
+        at::Tensor accum = empty_on(g, feature_size, at::kFloat);
+        accum.zero_();
+        roi_align_3d_backward(g.contiguous(), unpack(0).to(at::kFloat).contiguous(), accum, (int)g.size(2), (int)g.size(3), (int)g.size(4),
+                              spatial_scale, sampling_ratio, order);
+        return {accum.to(feature_dtype)};
+    }
+};
+
+at::Tensor roi_align_3d(const at::Tensor &features, const at::Tensor &rois, int out_d, int out_h, int out_w, float spatial_scale,
+                        int sampling_ratio, int order) {
+    at::Tensor output;
+    {
+        at::NoGradGuard no_grad;
+        output = features.new_empty({rois.size(0), features.size(1), out_d, out_h, out_w});
+        roi_align_3d_forward(features.contiguous(), rois.to(features.scalar_type()).contiguous(), output, out_d, out_h, out_w, spatial_scale,
+                             sampling_ratio, order);
+    }
+    if (fda_nodes::needs_node({features})) {
+        auto node = std::make_shared<RoIAlign3DBackward>();
+        node->feature_size = features.sizes().vec();
+        node->feature_dtype = features.scalar_type();
+        node->spatial_scale = spatial_scale;
+        node->sampling_ratio = sampling_ratio;
+        node->order = order;
+        node->save(0, rois);
+        fda_nodes::connect(node, output, torch::autograd::collect_next_edges(features));
+    }
+    return output;
 }
 
 at::Tensor nms_3d(const at::Tensor &dets, const at::Tensor &scores, const float threshold) {
@@ -279,6 +404,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.doc() = "B200 Flash Deformable 3D Attention (torch binding over the fda_b200 C ABI)";
     m.def("flash_deform_attn_forward", &flash_deform_attn_forward, "Flash Deformable 3D Attention forward (sm_100a)");
     m.def("flash_deform_attn_backward", &flash_deform_attn_backward, "Flash Deformable 3D Attention backward (sm_100a)");
+    m.def("flash_deform_attn", &flash_deform_attn, "differentiable Flash Deformable 3D Attention");
+    m.def("dcnv4", &dcnv4, "differentiable DCNv4-3D");
+    m.def("roi_align_3d", &roi_align_3d, "differentiable ROI-Align 3D");
     m.def("nms_3d", &nms_3d, "non-maximum suppression for 3d boxes (sm_100a)");
     m.def("roi_align_3d_forward", &roi_align_3d_forward, "ROI-Align 3D forward (sm_100a)");
     m.def("roi_align_3d_backward", &roi_align_3d_backward, "ROI-Align 3D backward (sm_100a)");

@@ -12,7 +12,6 @@ reference ``csrc/dcnv4.h:7-61``); the same two functions, with the same position
 from __future__ import annotations
 
 from torch.autograd import Function
-from torch.autograd.function import once_differentiable
 
 from ._extension import _C, _C_IMPORT_ERROR
 
@@ -28,21 +27,7 @@ class DCNv4Function(Function):
     remove_center, softmax)``; ``kernel`` .. ``dilation`` are (d, h, w) triples."""
 
     @staticmethod
-    def forward(ctx, value, p_offset, kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step=64,
-                remove_center=0, softmax=False):
-        ctx.cfg = (tuple(kernel), tuple(stride), tuple(pad), tuple(dilation), group, group_channels, float(offset_scale),
-                   im2col_step, int(remove_center), bool(softmax))
-        out = _ext().dcnv4_forward(value, p_offset, *kernel, *stride, *pad, *dilation, group, group_channels, float(offset_scale),
-                                   im2col_step, int(remove_center), 8, 0, bool(softmax))
-        ctx.save_for_backward(value, p_offset)
-        return out
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, grad_output):
-        value, p_offset = ctx.saved_tensors
-        kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step, remove_center, softmax = ctx.cfg
-        grad_value, grad_offset = _ext().dcnv4_backward(value, p_offset, *kernel, *stride, *pad, *dilation, group, group_channels,
-                                                        offset_scale, im2col_step, grad_output.contiguous(), remove_center, 8, 0,
-                                                        softmax)
-        return (grad_value, grad_offset) + (None,) * 10
+    def apply(value, p_offset, kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step=64, remove_center=0,
+              softmax=False):
+        return _ext().dcnv4(value, p_offset, kernel, stride, pad, dilation, group, group_channels, float(offset_scale), im2col_step,
+                            int(remove_center), bool(softmax))

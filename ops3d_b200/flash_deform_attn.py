@@ -15,13 +15,11 @@ and ``sampling_loc_attn`` (positions 0 and 3 of the 7 inputs), reference ``:68-1
 ``findspec`` / ``findspec_bwd`` are kept because callers import them (reference ``:26-62``; its
 wrapper test calls ``_C`` directly with their results).  They return the same numbers as the
 reference's but in O(sqrt(B*Q)) host time instead of a Python loop over every integer up to B*Q;
-the kernels treat the results as hints and ignore them.
+the kernels treat the results as hints and ignore them, so the operator itself does not compute them.
 """
 from __future__ import annotations
 
-import torch
 from torch.autograd import Function
-from torch.autograd.function import once_differentiable
 
 from ._extension import _C, _C_IMPORT_ERROR
 
@@ -71,38 +69,10 @@ def findspec_bwd(B, Q, G, C, max_tpb=256, max_mult=64):
 
 
 class FlashDeformAttnFunction(Function):
-    @staticmethod
-    def forward(ctx, value, value_spatial_shapes, value_level_start_index, sampling_loc_attn, im2col_step,
-                K=8, use_reg=True):
-        ext = _require_extension()
-        ctx.K = K
-        ctx.im2col_step = im2col_step
-
-        L = value_spatial_shapes.shape[0]
-        expected_last = L * K * 3 + L * K
-        if sampling_loc_attn.shape[-1] != expected_last:
-            raise ValueError(
-                "sampling_loc_attn last dimension ({}) does not match value_spatial_shapes level count "
-                "L={} and K={} (expected {})".format(sampling_loc_attn.shape[-1], L, K, expected_last)
-            )
-
-        B, Q, G, C = value.shape[0], sampling_loc_attn.shape[1], value.shape[2], value.shape[3]
-        d_stride, blockthread = findspec(B, Q, G, C)
-        ctx.d_stride_backward, ctx.blockthread_backward = findspec_bwd(B, Q, G, C)
-
-        output = ext.flash_deform_attn_forward(
-            value, value_spatial_shapes, value_level_start_index, sampling_loc_attn,
-            ctx.im2col_step, K, d_stride, blockthread, use_reg,
-        )
-        ctx.save_for_backward(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn)
-        return output
+    """The differentiable operator.  Forward, saved tensors and backward are a C++ graph node (``csrc/autograd_nodes.h``):
+    gradients reach ``value`` and ``sampling_loc_attn``, once (differentiating them raises)."""
 
     @staticmethod
-    @once_differentiable
-    def backward(ctx, grad_output):
-        value, value_spatial_shapes, value_level_start_index, sampling_loc_attn = ctx.saved_tensors
-        grad_value, grad_sampling_loc_attn = _require_extension().flash_deform_attn_backward(
-            value, value_spatial_shapes, value_level_start_index, sampling_loc_attn,
-            grad_output.contiguous(), ctx.im2col_step, ctx.K, ctx.d_stride_backward, ctx.blockthread_backward,
-        )
-        return grad_value, None, None, grad_sampling_loc_attn, None, None, None
+    def apply(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn, im2col_step, K=8, use_reg=True):
+        return _require_extension().flash_deform_attn(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn,
+                                                      im2col_step, K, use_reg)

@@ -112,7 +112,7 @@ size_t fda_backward_scratch_bytes(int batch, int num_value, int num_heads, int h
 
 /*
  * The cell-sorted backward (all points sorted by the cell they fall in; gathers and reductions once per run of equal
- * cells instead of once per point) applies to 16-bit values with 32 channels per head and enough points to pay for
+ * cells instead of once per point) applies to 16-bit values with 16, 32, 48 or 64 channels per head and enough points to pay for
  * its extra launches (FDA_BWD_SORT: 0 off, 1 by size, 2 always).  It needs more scratch than the slab-binned path:
  * fda_backward_sorted_scratch_bytes() (0 when it does not apply).  A caller that wants whichever path the library
  * prefers passes max(fda_backward_scratch_bytes, fda_backward_sorted_scratch_bytes) bytes; fda_backward_workspace_bytes

@@ -194,7 +194,8 @@ def forward_head_group(value, packed, K) -> int:
 
 
 def backward_path(value, packed, K) -> int:
-    """0 plain scatter kernel, 1 slab-binned largest level, 2 cell-sorted (what a call with scratch takes)."""
+    """0 plain scatter kernel, 1 slab-binned largest level, 2 cell-sorted, 3 cell-sorted with another number of channels
+    per head than 32 (what a call with scratch takes)."""
     B, N, G, D = value.shape
     return int(load().fda_backward_path(B, N, G, D, _levels(packed, K), packed.shape[1], K, DTYPE_CODE[value.dtype]))
 
@@ -206,11 +207,11 @@ def backward_touched_rows(value, packed, K) -> bool:
 
 
 def _scatter_launches(value, packed, K, first=True, last=True) -> int:
-    """Kernels of one scatter call that was given scratch: sorted = (count, 3 x scan, fill on the first launch of a
+    """Kernels of one scatter call that was given scratch: sorted = (clear, count, 3 x scan, fill on the first launch of a
     sequence) + walk (+ finalize on the last); binned = count, scan, fill, binned + plain; else the plain kernel."""
     path = backward_path(value, packed, K)
-    if path == 2:
-        return (5 if first else 0) + 1 + (1 if last else 0)
+    if path >= 2:
+        return (6 if first else 0) + 1 + (1 if last else 0)
     return 5 if path == 1 else 1
 
 

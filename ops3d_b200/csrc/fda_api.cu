@@ -63,10 +63,8 @@ fda::Config read_config() {
     c.peer_reduce_blocks = 32;
     c.fwd_head_groups = 1;
     c.sorted = 1;
-    c.sort_seg = 32;
     c.sort_grid_x = 0;
     c.touched = 1;
-    c.sort_ahead = 2;  // 2 / 3 / 4 with 3 / 2 / 2 resident blocks: 31.2 / 33.8 / 33.5 ms per full-size backward
     if (const char *e = std::getenv("FDA_L2_KEEP_FRACTION")) c.l2_keep_fraction = std::atof(e);
     if (c.l2_keep_fraction < 0) c.l2_keep_fraction = 0;
     if (const char *e = std::getenv("FDA_BINNING")) c.binning = std::atoi(e) != 0;
@@ -82,15 +80,8 @@ fda::Config read_config() {
     if (c.peer_reduce_blocks < 1) c.peer_reduce_blocks = 1;
     if (const char *e = std::getenv("FDA_FWD_HEAD_GROUPS")) c.fwd_head_groups = std::atoi(e);
     if (const char *e = std::getenv("FDA_BWD_SORT")) c.sorted = std::atoi(e);
-    if (const char *e = std::getenv("FDA_SORT_SEGMENT")) c.sort_seg = std::atoi(e);
-    c.sort_seg = (c.sort_seg + 3) & ~3;
-    if (c.sort_seg < 4) c.sort_seg = 4;
-    if (c.sort_seg > 256) c.sort_seg = 256;
     if (const char *e = std::getenv("FDA_SORT_GRID_X")) c.sort_grid_x = std::atoi(e);
     if (c.sort_grid_x < 0) c.sort_grid_x = 0;
-    if (const char *e = std::getenv("FDA_SORT_AHEAD")) c.sort_ahead = std::atoi(e);
-    if (c.sort_ahead < 2) c.sort_ahead = 2;
-    if (c.sort_ahead > 4) c.sort_ahead = 4;
     if (const char *e = std::getenv("FDA_BWD_TOUCHED")) c.touched = std::atoi(e);
     return c;
 }
@@ -249,36 +240,42 @@ size_t dalpha_plane_bytes(int B, int G, int L, int Q, int K, int pdt) {
     return round256((size_t)B * Q * G * L * K * sizeof(float));
 }
 
-// Cell-sorted backward: [counters [B*N*G]] [scan tile sums] [entries, 32 bytes per point] [results, 16 bytes per
-// point].  Zero when the path is switched off or the problem does not qualify: 16-bit
-// values with 32 channels per head only (rows of four lanes, which is what the walk's matrix instructions assume);
-// point ids and list positions are 32-bit; FDA_BWD_SORT=1 wants at least a few million points, below that the extra
-// launches cost more than they save.
+// Cell-sorted backward: [counters] [scan tile sums] [soft-max statistics, 8 bytes per row] [ranks, 4 bytes per point]
+// [entries, 32 bytes per point] [results, 16 bytes per point].  Zero when the path is switched off or the problem does not qualify: 16-bit values with
+// 16, 32, 48 or 64 channels per head only (whole k-steps of the walk's matrix products); point ids and list positions are
+// 32-bit; FDA_BWD_SORT=1 wants enough points, below that the extra launches cost more than they save.
+//
+// Whether it pays: measured per point, the plain scatter takes 0.12 / 0.155 / 0.375 ns with 2 / 4 / 8 lanes per row, the
+// sorted one 0.065 + 0.0009 D plus what a run costs (0.19 ns, 0.55 above 32 channels) over the points per run, about the
+// density of points per cell and head; its eight launches cost 70 us more than the three of the plain path.  At 32
+// channels that is 2.4 M points at a density of 4, 1.2 M at 16 (73728 cells: 398 -> 388 us at 2.4 M, 742 -> 583 at 4.7 M,
+// 1426 -> 990 at 9.4 M; 64 channels 955 -> 664, 1805 -> 945, 3526 -> 1477).
+bool sorted_pays(int D, double points, double density) {
+    const double plain = D <= 16 ? 0.12 : (D <= 32 ? 0.155 : 0.375);
+    const double sorted = 0.065 + 0.0009 * D + (D <= 32 ? 0.19 : 0.55) / density;
+    return points * (plain - sorted) > 70e3;
+}
 struct SortLayout {
-    size_t counters, tile_sums, entries, results, total;
-    unsigned long long bins, points;
+    size_t counters, tile_sums, stats, ranks, entries, results, total;
     unsigned int tiles;
 };
 SortLayout sort_layout(int B, int N, int G, int D, int L, int Q, int K, int vdt) {
     SortLayout s;
     std::memset(&s, 0, sizeof(s));
     if (g_config.sorted <= 0) return s;
-    if (vdt == FDA_DTYPE_F32 || D != 32) return s;
-    if (B <= 0 || N <= 0 || G <= 0 || L <= 0 || Q <= 0 || K <= 0 || G >= 65536) return s;
-    const unsigned long long bins = (unsigned long long)B * N * G;
-    const unsigned long long points = (unsigned long long)B * Q * G * L * K;
+    if (vdt == FDA_DTYPE_F32 || D % 16 != 0 || D > 64) return s;
+    if (B <= 0 || N <= 0 || G <= 0 || L <= 0 || Q <= 0 || K <= 0 || (long long)L * G > fda::kWalkRegions) return s;
+    // (W+1)(H+1)(D+1) bins per level and head: at most eight times its cells
+    const unsigned long long bins = 8ull * B * N * G + 1;
+    const unsigned long long points = (unsigned long long)B * Q * G * L * K, rows = (unsigned long long)B * Q * G;
     if (bins >= (1ull << 31) || points >= (1ull << 31)) return s;
-    // by size: a few million points at least (below that the five extra launches cost more than they save), and ten
-    // points per (cell, head) on average -- the walk gathers and reduces once per RUN of equal cells, so it needs runs.
-    // Measured per point of one rank's rows, full-size volume: sorted 0.143 / 0.170 ns at 24 / 12 points per cell and
-    // head, the slab-binned + plain kernels 0.18 ns whatever the density; the fit a + b / density crosses at 9.5.
-    if (g_config.sorted == 1 && (points < (4ull << 20) || (unsigned long long)Q * L * K < 10ull * N)) return s;
-    s.bins = bins;
-    s.points = points;
+    if (g_config.sorted == 1 && !sorted_pays(D, (double)points, (double)Q * L * K / N)) return s;
     s.tiles = (unsigned int)((bins + fda::kScanTile - 1) / fda::kScanTile);
     s.counters = 0;
     s.tile_sums = round256(bins * sizeof(unsigned int));
-    s.entries = s.tile_sums + round256((size_t)s.tiles * sizeof(unsigned int));
+    s.stats = s.tile_sums + round256((size_t)s.tiles * sizeof(unsigned int));
+    s.ranks = s.stats + round256(rows * sizeof(float2));
+    s.entries = s.ranks + round256(points * sizeof(float));
     s.results = s.entries + round256(points * 2 * sizeof(float4));
     s.total = s.results + round256(points * sizeof(float4));
     return s;
@@ -291,9 +288,10 @@ void attach_sorted(fda::Problem &p, const Shape &s, void *scratch, size_t scratc
     char *base = static_cast<char *>(scratch);
     p.sort_counters = reinterpret_cast<unsigned int *>(base + lay.counters);
     p.sort_tile_sums = reinterpret_cast<unsigned int *>(base + lay.tile_sums);
+    p.sort_stats = reinterpret_cast<float2 *>(base + lay.stats);
+    p.sort_ranks = reinterpret_cast<unsigned int *>(base + lay.ranks);
     p.sort_entries = reinterpret_cast<float4 *>(base + lay.entries);
     p.sort_results = reinterpret_cast<float4 *>(base + lay.results);
-    p.sort_seg = g_config.sort_seg;
     p.bin_allowed = 0;  // this layout replaces the binned one
     p.dalpha = nullptr;
 }
@@ -392,39 +390,35 @@ int launch_sorted(fda::Problem p, cudaStream_t st) {
     if constexpr (std::is_same<VT, float>::value) {
         return FDA_ERR_BAD_DTYPE;  // not reached: the layout is empty for fp32 values
     } else {
-        const unsigned long long bins = (unsigned long long)p.B * p.N * p.G;
-        const unsigned int tiles = (unsigned int)((bins + fda::kScanTile - 1) / fda::kScanTile);
         if (!p.resume) {
-            cudaError_t e = cudaMemsetAsync(p.sort_counters, 0, bins * sizeof(unsigned int), st);
-            if (e != cudaSuccess) return cuda_fail(e);
+            const unsigned long long bins = 8ull * p.B * p.N * p.G + 1;
+            const unsigned int tiles = (unsigned int)((bins + fda::kScanTile - 1) / fda::kScanTile);
+            const unsigned long long clear_blocks = (bins + 1023) / 1024;
+            fda::fda_sort_clear_kernel<<<(unsigned)(clear_blocks > 2368 ? 2368 : clear_blocks), 256, 0, st>>>(p);
             fda::Problem q = p;
             q.row_stride = padded_stride(4 * p.LK);
             const int threads = pick_threads(q, q.row_stride);
             const size_t smem = (size_t)(threads >> q.gs_log2) * q.row_stride * sizeof(float);
-            auto count = fda::fda_sort_pass_kernel<PT, false>;
-            auto fill = fda::fda_sort_pass_kernel<PT, true>;
+            auto count = fda::fda_sort_count_kernel<PT>;
             if (int rc = ensure_smem(reinterpret_cast<const void *>(count), smem)) return rc;
-            if (int rc = ensure_smem(reinterpret_cast<const void *>(fill), smem)) return rc;
             count<<<row_grid(q, threads), threads, smem, st>>>(q);
-            fda::fda_scan_tile_sums_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p.sort_counters, (size_t)bins, p.sort_tile_sums);
-            fda::fda_scan_spine_kernel<<<1, fda::kScanThreads, 0, st>>>(p.sort_tile_sums, tiles);
-            fda::fda_scan_apply_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p.sort_counters, (size_t)bins, p.sort_tile_sums);
+            fda::fda_scan_tile_sums_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p);
+            fda::fda_scan_spine_kernel<<<1, fda::kScanThreads, 0, st>>>(p);
+            fda::fda_scan_apply_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p);
+            auto fill = fda::fda_sort_fill_kernel<PT>;
+            if (int rc = ensure_smem(reinterpret_cast<const void *>(fill), smem)) return rc;
             fill<<<row_grid(q, threads), threads, smem, st>>>(q);
-            e = cudaGetLastError();
+            const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return cuda_fail(e);
         }
-        // shared memory of the walk: every warp's span of the list (32 bytes per entry) and every lane's ring of rows
-        constexpr int block = 128;
-        const int ahead = g_config.sort_ahead;
-        const size_t walk_smem = ((size_t)(block / 32) * 8 * (2 * (size_t)p.sort_seg + 1) + (size_t)ahead * fda::kWalkSlot * block) * 16;
-        int per_sm = (int)((size_t)227 * 1024 / (walk_smem + 1024));  // resident blocks: shared memory, then registers (3)
-        per_sm = per_sm > 3 ? 3 : (per_sm < 1 ? 1 : per_sm);
+        auto walk = p.D == 16 ? fda::fda_sorted_walk_kernel<VT, 1> : (p.D == 32 ? fda::fda_sorted_walk_kernel<VT, 2>
+                    : (p.D == 48 ? fda::fda_sorted_walk_kernel<VT, 3> : fda::fda_sorted_walk_kernel<VT, 4>));
+        const size_t walk_smem = sizeof(fda::WalkShared);
+        if (int rc = ensure_smem(reinterpret_cast<const void *>(walk), walk_smem)) return rc;
+        const int per_sm = p.D <= 32 ? 4 : (p.D == 48 ? 3 : 2);  // resident blocks, by registers
         int gx = g_config.sort_grid_x;
         if (gx <= 0) gx = (per_sm * sm_count() + p.B - 1) / p.B;
-        auto walk = ahead == 2 ? fda::fda_sorted_walk_kernel<VT, block, 3, 2>
-                               : (ahead == 3 ? fda::fda_sorted_walk_kernel<VT, block, 3, 3> : fda::fda_sorted_walk_kernel<VT, block, 3, 4>);
-        if (int rc = ensure_smem(reinterpret_cast<const void *>(walk), walk_smem)) return rc;
-        walk<<<dim3((unsigned)gx, (unsigned)p.B, 1), block, walk_smem, st>>>(p);
+        walk<<<dim3((unsigned)gx, (unsigned)p.B, 1), fda::kWalkWarps * 32, walk_smem, st>>>(p);
         if (p.finalize) {
             fda::Problem q = p;
             q.row_stride = padded_stride(5 * p.LK);
@@ -566,7 +560,8 @@ size_t fda_backward_sorted_scratch_bytes(int batch, int num_value, int num_heads
 
 int fda_backward_path(int batch, int num_value, int num_heads, int head_dim, int num_levels, int num_query, int num_points,
                       int value_dtype) {
-    if (sort_layout(batch, num_value, num_heads, head_dim, num_levels, num_query, num_points, value_dtype).total) return 2;
+    if (sort_layout(batch, num_value, num_heads, head_dim, num_levels, num_query, num_points, value_dtype).total)
+        return head_dim == 32 ? 2 : 3;
     return bin_scratch_bytes(batch, num_value, num_heads, head_dim, num_query, num_points) ? 1 : 0;
 }
 

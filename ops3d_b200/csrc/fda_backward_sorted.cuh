@@ -1,28 +1,25 @@
-// Cell-sorted backward for 16-bit values with 32 channels per head (rows of exactly four lanes).
+// Cell-sorted backward for 16-bit values with 16, 32, 48 or 64 channels per head.
 //
 // Every sampling point of a call is sorted by the cell of the pyramid it falls in (and its head); the sorted list is
-// then walked so that consecutive points read the same eight value rows and add into the same eight rows of the fp32
-// gradient image.  A lane group keeps both sets of rows in registers for as long as the cell does not change: eight
-// gathers and eight reductions per RUN of equal cells instead of per POINT.
+// then walked run by run of equal cells.  The eight value rows of a cell are read, and its eight rows of the fp32
+// gradient image added to, once per RUN instead of once per POINT, and inside a run everything is small matrix products.
 //
 // Why: a (cell, head) row receives Q*K / cells contributions (9 / 73 / 584 on a 32x64x256 / 16x32x128 / 8x16x64
 // pyramid with K = 8 points per level and one query per cell), and the plain and the slab-binned kernels are bound by
 // exactly those gathers and reductions (the request path from the SMs to L2), not by HBM.
 //
-//   fda_sort_pass_kernel<count> rows staged like in fda_backward_kernel; one counter per (batch, cell, head)
+//   fda_sort_clear_kernel     zeroes the counters, one per (batch, level, head, base cell)
+//   fda_sort_count_kernel     rows staged like in fda_backward_kernel; rank of every point inside its bin (the one atomic
+//                             per point), soft-max statistics of the row
 //   fda_scan_*                exclusive scan of the counters (three small kernels, no waiting between blocks)
-//   fda_sort_pass_kernel<fill> soft-max of the row; position = atomicAdd(counter of the point's bin); files the point
-//                             there as one 32-byte record (one 256-bit store)
-//   fda_sorted_walk_kernel    grid (x, batch): lane groups walk segments of the sorted list of the launch's levels.
-//                             Everything a point needs from global memory (its grad_output row, and the eight value
-//                             rows when it starts a run) is copied asynchronously into shared memory a few points
-//                             ahead.  The eight dot products <value row, grad_output row> of a point are warp-level
-//                             matrix instructions; the gradient image rows are accumulated in registers and sent with
-//                             one reduction per corner when the run ends.  Writes {d/dx, d/dy, d/dz, dalpha} of the
-//                             point into a row-ordered array (a scattered 16-byte store: the walk has DRAM bandwidth
-//                             to spare, the pass that follows would pay 64 bytes per random 16-byte read).
-//   fda_sort_finalize_kernel  per row: its points' results (contiguous), soft-max backward, finished row of
-//                             grad_sampling_loc_attn, coalesced
+//   fda_sort_fill_kernel      position = start of the bin + rank; files the point there as one 32-byte record
+//   fda_sorted_walk_kernel    grid (x, batch): warps walk spans of the list of the launch's levels; the points' results
+//                             {d/dx, d/dy, d/dz, dalpha} in list order
+//   fda_sort_finalize_kernel  per row: its points' results, soft-max backward, finished row of grad_sampling_loc_attn
+//
+// Bins are ordered (batch, level, head, cell): a region of one head reads one head's grad_output rows at random.  A base
+// cell may be -1 along an axis (only its upper corners lie inside), so a level of W x H x D cells has (W+1)(H+1)(D+1)
+// bins: every point of a bin has the same eight corners.
 //
 // A launch over a level range that is not the first of a sequence (`resume`) re-uses the list made by the first.
 // Nothing here waits on another block.  No counterpart in the reference (its backward is one thread group per query
@@ -37,31 +34,39 @@ constexpr int kScanItems = 8;                         // counters per thread of 
 constexpr int kScanThreads = 1024;
 constexpr int kScanTile = kScanItems * kScanThreads;  // counters per scan block
 constexpr unsigned int kNoPosition = 0xffffffffu;     // a point without a corner inside its level
-constexpr int kWalkSlot = 9;                          // 16-byte vectors per lane and point: grad_output row + eight value rows
 
-// What the count and the fill pass agree on: bin and geometry tags of a point from its voxel coordinates.
-struct SortTag {
-    bool ok;             // some corner lies inside the level
-    unsigned int bin;    // (first cell of the level + base cell clamped to the level) * G + head
-    unsigned int in8;    // bit n: corner n = dz*4 + dy*2 + dx lies inside the level
-    unsigned int off0;   // element offset of the (unclamped) base corner inside the level, modulo 2^32
+// Bins of one batch element: level l's start at first[l], head g's inside it at g * cells[l].  first[L] = all of them.
+struct SortBins {
+    unsigned int first[kMaxLevels + 1], cells[kMaxLevels];
 };
-__device__ __forceinline__ SortTag sort_tag_of(const LevelGeom &lv, int G, int GD, unsigned int g, float xv, float yv, float zv) {
-    SortTag t;
+__device__ __forceinline__ void build_sort_bins(SortBins &s, const int64_t *shapes, int L, int G) {
+    unsigned int at = 0;
+    for (int l = 0; l < L; ++l) {
+        s.first[l] = at;
+        s.cells[l] = (unsigned int)(shapes[3 * l] + 1) * (unsigned int)(shapes[3 * l + 1] + 1) * (unsigned int)(shapes[3 * l + 2] + 1);
+        at += s.cells[l] * (unsigned int)G;
+    }
+    s.first[L] = at;
+}
+
+// Base cell of a point from its normalised coordinates, and whether any corner lies inside the level.
+struct BaseCell {
+    bool ok;
+    int x, y, z;        // in [-1, size-1] when ok
+    float fx, fy, fz;   // fraction towards the upper corner: upper weight f, lower 1 - f (in range the same value as (floor + 1) - v)
+};
+__device__ __forceinline__ BaseCell base_cell(const LevelGeom &lv, float x, float y, float z) {
+    const float xv = unnormalize(x, lv.fW), yv = unnormalize(y, lv.fH), zv = unnormalize(z, lv.fD);
     const float xf = floorf(xv), yf = floorf(yv), zf = floorf(zv);
+    BaseCell c;
     // an axis has a corner in range iff floor in [-1, size-1]; written so that NaN fails
-    t.ok = (xf >= -1.f) && (xf <= lv.fW - 1.0f) && (yf >= -1.f) && (yf <= lv.fH - 1.0f) && (zf >= -1.f) && (zf <= lv.fD - 1.0f);
-    t.bin = 0u; t.in8 = 0u; t.off0 = 0u;
-    if (!t.ok) return t;
-    const int x0 = (int)xf, y0 = (int)yf, z0 = (int)zf;  // in [-1, size-1]
-    const unsigned int cx = x0 < 0 ? 0u : (unsigned int)x0, cy = y0 < 0 ? 0u : (unsigned int)y0, cz = z0 < 0 ? 0u : (unsigned int)z0;
-    t.bin = ((unsigned int)lv.start + (cz * (unsigned int)lv.H + cy) * (unsigned int)lv.W + cx) * (unsigned int)G + g;
-    const unsigned int mx = (unsigned int)(x0 >= 0) | (unsigned int)(x0 + 1 < lv.W) << 1;        // corners dx = 0, 1
-    const unsigned int mxy = (y0 >= 0 ? mx : 0u) | (y0 + 1 < lv.H ? mx << 2 : 0u);              // dy*2 + dx
-    t.in8 = (z0 >= 0 ? mxy : 0u) | (z0 + 1 < lv.D ? mxy << 4 : 0u);                             // dz*4 + dy*2 + dx
-    const uint32_t sx = (uint32_t)GD, sy = (uint32_t)lv.W * sx, sz = (uint32_t)lv.H * sy;
-    t.off0 = (uint32_t)z0 * sz + (uint32_t)y0 * sy + (uint32_t)x0 * sx;  // wraps for index -1; + stride wraps back
-    return t;
+    c.ok = (xf >= -1.f) && (xf <= lv.fW - 1.0f) && (yf >= -1.f) && (yf <= lv.fH - 1.0f) && (zf >= -1.f) && (zf <= lv.fD - 1.0f);
+    c.x = c.ok ? (int)xf : 0; c.y = c.ok ? (int)yf : 0; c.z = c.ok ? (int)zf : 0;
+    c.fx = __fsub_rn(xv, xf); c.fy = __fsub_rn(yv, yf); c.fz = __fsub_rn(zv, zf);
+    return c;
+}
+__device__ __forceinline__ unsigned int bin_of(const LevelGeom &lv, const BaseCell &c) {  // inside its level and head
+    return ((unsigned int)(c.z + 1) * (unsigned int)(lv.H + 1) + (unsigned int)(c.y + 1)) * (unsigned int)(lv.W + 1) + (unsigned int)(c.x + 1);
 }
 
 // One 32-byte list record as ONE streaming store (sm_100: 256-bit vector store); `rec` is 32-byte aligned.
@@ -70,13 +75,100 @@ __device__ __forceinline__ void store_record(float4 *rec, const float4 &a, const
                  "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w) : "memory");
 }
 
-// kFill = false: counts the points of every bin.  kFill = true: the counters hold the exclusive scan; files the points.
-template <typename PT, bool kFill>
-__global__ void __launch_bounds__(kThreads) fda_sort_pass_kernel(const Problem p) {
+__global__ void __launch_bounds__(256) fda_sort_clear_kernel(const Problem p) {
+    __shared__ SortBins bins;
+    if (threadIdx.x == 0) build_sort_bins(bins, p.shapes, p.L, p.G);
+    __syncthreads();
+    const size_t n = (size_t)bins.first[p.L] * p.B + 1;  // one more: after the scan it holds the length of the list
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; 4 * i < n; i += (size_t)gridDim.x * blockDim.x) {
+        if (4 * i + 4 <= n) reinterpret_cast<uint4 *>(p.sort_counters)[i] = make_uint4(0u, 0u, 0u, 0u);
+        else
+            for (size_t k = 4 * i; k < n; ++k) p.sort_counters[k] = 0u;
+    }
+}
+
+// Rank of every point inside its bin, in row order ([row][L*K], kNoPosition for a point that is not filed), and the
+// soft-max statistics {max, 1 / sum} of every row.
+template <typename PT>
+__global__ void __launch_bounds__(kThreads) fda_sort_count_kernel(const Problem p) {
     __shared__ LevelGeom geom[kMaxLevels];
+    __shared__ SortBins bins;
     extern __shared__ __align__(16) float smem_tile[];
     const int tid = threadIdx.x;
-    if (tid == 0) build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, false, 0ull);
+    if (tid == 0) {
+        build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, false, 0ull);
+        build_sort_bins(bins, p.shapes, p.L, p.G);
+    }
+    const int b = blockIdx.y;
+    const int gs = 1 << p.gs_log2;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int lane_c = tid & (gs - 1);
+    const int rows_per_block = (int)blockDim.x >> p.gs_log2;
+    const int rows_per_warp = 32 >> p.gs_log2;
+    const int row = blockIdx.x * rows_per_block + (tid >> p.gs_log2);
+    const bool row_ok = row < p.rows_per_b;
+    const int LK = p.LK;
+    const int first = blockIdx.x * rows_per_block + warp * rows_per_warp;
+    float *wtile = smem_tile + warp * rows_per_warp * p.row_stride;
+    int nrows = p.rows_per_b - first;
+    nrows = nrows < 0 ? 0 : (nrows > rows_per_warp ? rows_per_warp : nrows);
+    stage_rows<PT>(static_cast<const PT *>(p.packed) + ((size_t)b * p.rows_per_b + first) * (size_t)(4 * LK), wtile, nrows,
+                   LK, p.row_stride, lane);
+    __syncthreads();  // level table and this warp's tile visible
+    float *trow = wtile + (lane >> p.gs_log2) * p.row_stride;
+    const unsigned int g = row_ok ? (unsigned int)(row % p.G) : 0u;
+    unsigned int *counters = p.sort_counters + (size_t)b * bins.first[p.L];
+    float m = -INFINITY;
+    for (int i = lane_c; i < LK; i += gs) m = fmaxf(m, row_ok ? trow[3 * LK + i] : 0.f);
+    for (int mask = gs >> 1; mask > 0; mask >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, mask));
+    float s = 0.f;
+    for (int i = lane_c; i < LK; i += gs) s += row_ok ? __expf(trow[3 * LK + i] - m) : 0.f;
+    for (int mask = gs >> 1; mask > 0; mask >>= 1) s += __shfl_xor_sync(0xffffffffu, s, mask);
+    if (row_ok && lane_c == 0) p.sort_stats[(size_t)b * p.rows_per_b + row] = make_float2(m, 1.0f / s);
+    // Eight points at a time: all requests go out before the first answer is needed.  The ranks take the place of the
+    // logits in the tile (a lane overwrites only slots it owns).
+    constexpr int kBatch = 8;
+    for (int i0 = lane_c; row_ok && i0 < LK; i0 += kBatch * gs) {
+        unsigned int rank[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int i = i0 + u * gs;
+            rank[u] = kNoPosition;
+            if (i < LK) {
+                const int l = (i >> 2) >> p.k_shift;
+                const LevelGeom lv = geom[l];
+                const BaseCell c = base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2]);
+                if (c.ok) rank[u] = atomicAdd(counters + bins.first[l] + g * bins.cells[l] + bin_of(lv, c), 1u);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int i = i0 + u * gs;
+            if (i < LK) trow[3 * LK + i] = __uint_as_float(rank[u]);
+        }
+    }
+    __syncwarp();
+    float *dst = reinterpret_cast<float *>(p.sort_ranks) + ((size_t)b * p.rows_per_b + first) * (size_t)LK;
+    const float inv_vec = 4.0f / (float)LK;
+    for (int v = lane; v < nrows * (LK >> 2); v += 32) {
+        const int r = row_of_vector(v, inv_vec);
+        const int c = (v - r * (LK >> 2)) * 4;
+        *reinterpret_cast<float4 *>(dst + (size_t)v * 4) = *reinterpret_cast<const float4 *>(wtile + r * p.row_stride + 3 * LK + c);
+    }
+}
+
+// Files every point at its position: start of its bin + rank, so nothing here depends on the answer of an atomic.  Rows
+// are staged like in the count pass; the position takes the place of the rank.
+template <typename PT>
+__global__ void __launch_bounds__(kThreads) fda_sort_fill_kernel(const Problem p) {
+    __shared__ LevelGeom geom[kMaxLevels];
+    __shared__ SortBins bins;
+    extern __shared__ __align__(16) float smem_tile[];
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, false, 0ull);
+        build_sort_bins(bins, p.shapes, p.L, p.G);
+    }
     const int b = blockIdx.y;
     const int gs = 1 << p.gs_log2;
     const int lane = tid & 31, warp = tid >> 5;
@@ -95,61 +187,40 @@ __global__ void __launch_bounds__(kThreads) fda_sort_pass_kernel(const Problem p
     if (row >= p.rows_per_b) return;
     const float *trow = wtile + (lane >> p.gs_log2) * p.row_stride;
     const unsigned int g = (unsigned int)(row % p.G);
-    unsigned int *counters = p.sort_counters + (size_t)b * ((size_t)p.N * p.G);
-    float m = 0.f, inv = 0.f;
-    if (kFill) {
-        m = -INFINITY;
-        for (int j = 0; j < (LK >> 2); ++j) {
-            const float4 lg = *reinterpret_cast<const float4 *>(trow + 3 * LK + 4 * j);
-            m = fmaxf(m, fmaxf(fmaxf(lg.x, lg.y), fmaxf(lg.z, lg.w)));
-        }
-        float s = 0.f;
-        for (int j = 0; j < (LK >> 2); ++j) {
-            const float4 lg = *reinterpret_cast<const float4 *>(trow + 3 * LK + 4 * j);
-            s += __expf(lg.x - m) + __expf(lg.y - m) + __expf(lg.z - m) + __expf(lg.w - m);
-        }
-        inv = 1.0f / s;
-    }
     const size_t rowg = (size_t)b * p.rows_per_b + row;
-    // Eight points at a time: all position requests go out before the first answer is needed.  Only the positions are
-    // kept across the two loops; recomputing a point's coordinates and tags is cheaper than the registers that would
-    // hold them (occupancy is what hides the latency of the requests).
-    constexpr int kBatch = 8;
+    const unsigned int *starts = p.sort_counters + (size_t)b * bins.first[p.L];
+    unsigned int *ranks = p.sort_ranks + rowg * (size_t)LK;
+    const float2 stats = __ldg(p.sort_stats + rowg);
+    constexpr int kBatch = 4;  // the starts of four points are requested before the first is used
     for (int i0 = lane_c; i0 < LK; i0 += kBatch * gs) {
-        unsigned int pos[kBatch];
+        unsigned int pos[kBatch], start[kBatch];
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
             const int i = i0 + u * gs;
-            pos[u] = kNoPosition;
-            if (i < LK) {
-                const LevelGeom lv = geom[(i >> 2) >> p.k_shift];
-                const SortTag tag = sort_tag_of(lv, p.G, p.GD, g, unnormalize(trow[3 * i], lv.fW), unnormalize(trow[3 * i + 1], lv.fH),
-                                                unnormalize(trow[3 * i + 2], lv.fD));
-                if (tag.ok) {
-                    if (kFill) pos[u] = atomicAdd(counters + tag.bin, 1u);
-                    else atomicAdd(counters + tag.bin, 1u);
-                }
+            pos[u] = i < LK ? ranks[i] : kNoPosition;
+            start[u] = 0u;
+            if (pos[u] != kNoPosition) {
+                const int l = (i >> 2) >> p.k_shift;
+                const LevelGeom lv = geom[l];
+                start[u] = __ldg(starts + bins.first[l] + g * bins.cells[l] + bin_of(lv, base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2])));
             }
         }
-        if (kFill) {
 #pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                const int i = i0 + u * gs;
-                if (i < LK) {
-                    if (pos[u] != kNoPosition) {
-                        const int l = (i >> 2) >> p.k_shift;
-                        const LevelGeom lv = geom[l];
-                        const float xv = unnormalize(trow[3 * i], lv.fW), yv = unnormalize(trow[3 * i + 1], lv.fH),
-                                    zv = unnormalize(trow[3 * i + 2], lv.fD);
-                        const SortTag tag = sort_tag_of(lv, p.G, p.GD, g, xv, yv, zv);
-                        // one 32-byte record = one whole sector (no read-modify-write behind the store)
-                        const unsigned int meta = (unsigned int)l | (g << 4) | (tag.in8 << 20);
-                        store_record(p.sort_entries + 2 * (size_t)pos[u], make_float4(xv, yv, zv, __expf(trow[3 * LK + i] - m) * inv),
-                                     make_float4(__uint_as_float((unsigned int)rowg), __uint_as_float(meta), __uint_as_float(tag.off0),
-                                                 __uint_as_float((unsigned int)i)));
-                    }
-                }
-            }
+        for (int u = 0; u < kBatch; ++u) {
+            const int i = i0 + u * gs;
+            if (pos[u] == kNoPosition) continue;
+            const LevelGeom lv = geom[(i >> 2) >> p.k_shift];
+            const BaseCell c = base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2]);
+            const uint32_t sx = (uint32_t)p.GD, sy = (uint32_t)lv.W * sx, sz = (uint32_t)lv.H * sy;
+            const unsigned int mx = (unsigned int)(c.x >= 0) | (unsigned int)(c.x + 1 < lv.W) << 1;    // corners dx = 0, 1
+            const unsigned int mxy = (c.y >= 0 ? mx : 0u) | (c.y + 1 < lv.H ? mx << 2 : 0u);          // dy*2 + dx
+            const unsigned int in8 = (c.z >= 0 ? mxy : 0u) | (c.z + 1 < lv.D ? mxy << 4 : 0u);        // dz*4 + dy*2 + dx
+            const uint32_t off0 = (uint32_t)c.z * sz + (uint32_t)c.y * sy + (uint32_t)c.x * sx;      // wraps for index -1; + stride wraps back
+            const unsigned int at = start[u] + pos[u];
+            // one 32-byte record = one whole sector (no read-modify-write behind the store)
+            store_record(p.sort_entries + 2 * (size_t)at, make_float4(c.fx, c.fy, c.fz, __expf(trow[3 * LK + i] - stats.x) * stats.y),
+                         make_float4(__uint_as_float((unsigned int)rowg), 0.f, __uint_as_float(off0), __uint_as_float(in8)));
+            ranks[i] = at;
         }
     }
 }
@@ -183,8 +254,18 @@ __device__ __forceinline__ unsigned int block_exclusive_scan(unsigned int v, uns
     return r;
 }
 
-__global__ void __launch_bounds__(kScanThreads) fda_scan_tile_sums_kernel(const unsigned int *__restrict__ data, size_t n,
-                                                                         unsigned int *__restrict__ tile_sums) {
+// The host sizes the counters for the most bins a volume of N cells can have; the kernels find the real number.
+__device__ __forceinline__ size_t counters_of(const Problem &p) {
+    SortBins bins;
+    build_sort_bins(bins, p.shapes, p.L, p.G);
+    return (size_t)bins.first[p.L] * p.B + 1;
+}
+
+__global__ void __launch_bounds__(kScanThreads) fda_scan_tile_sums_kernel(const Problem p) {
+    const unsigned int *__restrict__ data = p.sort_counters;
+    unsigned int *__restrict__ tile_sums = p.sort_tile_sums;
+    const size_t n = counters_of(p);
+    if ((size_t)blockIdx.x * kScanTile >= n) return;
     __shared__ unsigned int warp_sums[33];
     const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
     unsigned int s = 0;
@@ -195,7 +276,9 @@ __global__ void __launch_bounds__(kScanThreads) fda_scan_tile_sums_kernel(const 
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kScanThreads) fda_scan_spine_kernel(unsigned int *tile_sums, unsigned int tiles) {
+__global__ void __launch_bounds__(kScanThreads) fda_scan_spine_kernel(const Problem p) {
+    unsigned int *tile_sums = p.sort_tile_sums;
+    const unsigned int tiles = (unsigned int)((counters_of(p) + kScanTile - 1) / kScanTile);
     __shared__ unsigned int warp_sums[33];
     unsigned int carry = 0;
     for (unsigned int base = 0; base < tiles; base += kScanThreads) {  // uniform trip count
@@ -208,8 +291,11 @@ __global__ void __launch_bounds__(kScanThreads) fda_scan_spine_kernel(unsigned i
     }
 }
 
-__global__ void __launch_bounds__(kScanThreads) fda_scan_apply_kernel(unsigned int *__restrict__ data, size_t n,
-                                                                     const unsigned int *__restrict__ tile_offsets) {
+__global__ void __launch_bounds__(kScanThreads) fda_scan_apply_kernel(const Problem p) {
+    unsigned int *__restrict__ data = p.sort_counters;
+    const unsigned int *__restrict__ tile_offsets = p.sort_tile_sums;
+    const size_t n = counters_of(p);
+    if ((size_t)blockIdx.x * kScanTile >= n) return;
     __shared__ unsigned int warp_sums[33];
     const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
     unsigned int v[kScanItems];
@@ -229,10 +315,6 @@ __global__ void __launch_bounds__(kScanThreads) fda_scan_apply_kernel(unsigned i
 }
 
 // ---- the walk over the sorted list ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned int)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-// the same through L2 only: for rows that are read once (they would only push re-used rows out of L1)
 __device__ __forceinline__ void cp_async16_once(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned int)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
 }
@@ -241,233 +323,384 @@ template <int kPending> __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
-// <value row, grad_output row> as warp-level matrix instructions: the four lanes of row group g hold row g of the A
-// fragment (their 16-byte vectors of a value row ARE the fragment, no unpacking) and column g of the B fragment (their
-// vectors of the grad_output row), so D[g][g] of an m16n8k16 product is the dot product over 16 channels, summed over
-// the group's lanes.  Two corners ride in one instruction (fragment rows g and g + 8), two instructions cover the 32
-// channels.  The other 7/8 of each product (row g against the grad_output of the other groups) is discarded.
-// `first`: d = A * B (zero accumulator input); `mma`: c += A * B.
-#define FDA_MMA_DOT(TYPES)                                                                                                             \
-    static __device__ __forceinline__ void first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,      \
-                                                 uint32_t b1) {                                                                         \
-        asm("mma.sync.aligned.m16n8k16.row.col." TYPES " {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"           \
-            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));       \
-    }                                                                                                                                   \
-    static __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,        \
-                                               uint32_t b1) {                                                                           \
-        asm("mma.sync.aligned.m16n8k16.row.col." TYPES " {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"               \
-            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));                 \
+// Warp-level matrix products in the value dtype with fp32 accumulators, and the split of two fp32 weights into three
+// 16-bit terms (hi + mid + lo: 24 significant bits and more, so nothing of an fp32 weight is lost).
+template <typename VT> struct WarpMma;
+#define FDA_WARP_MMA(TYPE)                                                                                                          \
+    static __device__ __forceinline__ void k16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,       \
+                                               uint32_t b1) {                                                                        \
+        asm("mma.sync.aligned.m16n8k16.row.col.f32." TYPE "." TYPE ".f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};" \
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));               \
+    }                                                                                                                                \
+    static __device__ __forceinline__ void k8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {                               \
+        asm("mma.sync.aligned.m16n8k8.row.col.f32." TYPE "." TYPE ".f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"         \
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));                                          \
     }
-template <typename VT> struct MmaDot;
-template <> struct MmaDot<__nv_bfloat16> { FDA_MMA_DOT("f32.bf16.bf16.f32") };
-template <> struct MmaDot<__half> { FDA_MMA_DOT("f32.f16.f16.f32") };
-#undef FDA_MMA_DOT
-
-// Work unit: a segment of S consecutive list entries per lane group; the groups of a warp take consecutive segments, so a
-// warp's share of one round is one contiguous span of the list, which it first copies to shared memory (coalesced).
-// Shared memory: [warps][span] 32-byte records, then per lane a ring of kAhead slots of kWalkSlot 16-byte vectors.
-// kAhead: points whose rows are in flight per lane.
-template <typename VT, int kBlock, int kMinBlocks, int kAhead>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) fda_sorted_walk_kernel(const Problem p) {
-    static_assert(Vec16<VT>::kCPL == 8, "16-bit value dtypes only");
-    constexpr unsigned int kNoRun = 0xffffffffu;
-    __shared__ LevelGeom geom[kMaxLevels];
-    __shared__ unsigned int s_begin, s_end;
-    extern __shared__ __align__(16) float smem_tile[];
-    const int tid = threadIdx.x;
-    const int b = blockIdx.y;
-    if (tid == 0) {
-        build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, true, p.l2_keep_bytes);
-        // The launch's levels are a contiguous range, and the list is ordered (batch, level, cell, head): its entries
-        // are one contiguous span per batch element.  After the fill pass a counter holds the END of its bin, i.e.
-        // the start of the next one.
-        const int lb = __ffs(p.level_mask) - 1, le = 32 - __clz(p.level_mask);
-        const unsigned long long NG = (unsigned long long)p.N * p.G;
-        const unsigned long long kf = (unsigned long long)b * NG + (unsigned long long)p.lsi[lb] * p.G;
-        const unsigned long long ke = (unsigned long long)b * NG + (unsigned long long)(le < p.L ? p.lsi[le] : (long long)p.N) * p.G;
-        s_begin = kf ? p.sort_counters[kf - 1] : 0u;
-        s_end = ke ? p.sort_counters[ke - 1] : 0u;
+template <> struct WarpMma<__nv_bfloat16> {
+    FDA_WARP_MMA("bf16")
+    static constexpr float kScale = 1.0f, kUnscale = 1.0f;
+    static __device__ __forceinline__ uint32_t take(float &w0, float &w1) {  // rounds the pair to 16 bits, leaves the remainders
+        const __nv_bfloat162 h = __floats2bfloat162_rn(w0, w1);
+        const uint32_t r = *reinterpret_cast<const uint32_t *>(&h);
+        w0 -= __uint_as_float(r << 16);
+        w1 -= __uint_as_float(r & 0xffff0000u);
+        return r;
     }
-    __syncthreads();
-    const unsigned int e_begin = s_begin, e_end = s_end;
-    if (e_end <= e_begin) return;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int tig = lane & 3, grp = lane >> 2;  // lane inside the row group, row group inside the warp
-    const int owner = grp >> 1;                 // the lane of the group that ends up with D[g][g] (c[g & 1]) and D[g + 8][g] (c[2 + (g & 1)])
-    const bool odd = grp & 1;
-    const unsigned int warps_per_block = blockDim.x >> 5;
-    const unsigned int S = (unsigned int)p.sort_seg;
-    const unsigned int span = S * 8u;  // list entries a warp takes at a time
-    const unsigned int nspan = (e_end - e_begin + span - 1) / span;
-    const uint64_t pol_keep = l2_policy_evict_last(), pol_stream = l2_policy_evict_first();
-    const VT *go_base = static_cast<const VT *>(p.grad_out) + (size_t)tig * 8;
-    const VT *value_b = static_cast<const VT *>(p.value) + (size_t)b * p.N * p.GD + (size_t)tig * 8;
-    float *image_b = p.accum + (size_t)b * p.N * p.GD + (size_t)tig * 8;
-    // a group's segment starts (2 * S + 1) vectors after its neighbour's: the eight groups of a warp read their records
-    // from eight different bank quads
-    const unsigned int seg_stride = 2u * S + 1u;
-    float4 *ent_s = reinterpret_cast<float4 *>(smem_tile) + (size_t)warp * 8u * seg_stride;
-    uint4 *ring = reinterpret_cast<uint4 *>(smem_tile) + (size_t)warps_per_block * 8u * seg_stride + tid;  // vector v of slot k: ring[(k * kWalkSlot + v) * blockDim.x]
+};
+template <> struct WarpMma<__half> {
+    FDA_WARP_MMA("f16")
+    // weights are in [0, 1]: scaled up, the smallest term of a weight of 1e-6 is still above fp16's subnormal step
+    static constexpr float kScale = 32768.0f, kUnscale = 1.0f / 32768.0f;
+    static __device__ __forceinline__ uint32_t take(float &w0, float &w1) {
+        const __half2 h = __floats2half2_rn(w0, w1);
+        const float2 f = __half22float2(h);
+        w0 -= f.x;
+        w1 -= f.y;
+        return *reinterpret_cast<const uint32_t *>(&h);
+    }
+};
+#undef FDA_WARP_MMA
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+    uint32_t r;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
 
-    float acc[8][8];
-    uint4 va[8];                                   // the run's eight value rows (this lane's channels), zero where outside the level
-    unsigned int run_off = 0u, run_meta = kNoRun;  // base offset of the run's cell; level | head << 4 | corner mask << 20
-
-    // sends the run's eight image rows to memory and clears them
-    auto flush = [&]() {
-        if (run_meta != kNoRun) {
-            const LevelGeom lv = geom[run_meta & 15u];
-            const uint32_t sx = (uint32_t)p.GD, sy = (uint32_t)lv.W * sx, sz = (uint32_t)lv.H * sy;
-            float *img = image_b + (size_t)lv.start * p.GD + (size_t)((run_meta >> 4) & 0xffffu) * p.D;
-            const uint64_t pol = (lv.keep & 2) ? pol_keep : pol_stream;
-            const unsigned int in8 = run_meta >> 20;
+// A lane's quarter of a head row of D = 16 * KS channels: channels tig * D/4 ... as 2 * KS words.
+template <int KS> struct RowWords {
+    uint32_t w[2 * KS];
+    __device__ __forceinline__ void zero() {
 #pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                const bool in = (in8 >> n) & 1u;
-                if (in) {
-                    float *dst = img + (uint32_t)(run_off + ((n & 4) ? sz : 0u) + ((n & 2) ? sy : 0u) + ((n & 1) ? sx : 0u));
-                    red_add_f32x4_hint(dst, acc[n][0], acc[n][1], acc[n][2], acc[n][3], pol);
-                    red_add_f32x4_hint(dst + 4, acc[n][4], acc[n][5], acc[n][6], acc[n][7], pol);
-                }
+        for (int i = 0; i < 2 * KS; ++i) w[i] = 0u;
+    }
+    __device__ __forceinline__ void load(const void *p) {
+        if constexpr (KS % 2 == 0) {
+#pragma unroll
+            for (int i = 0; i < KS / 2; ++i) {
+                const uint4 r = __ldg(static_cast<const uint4 *>(p) + i);
+                w[4 * i] = r.x; w[4 * i + 1] = r.y; w[4 * i + 2] = r.z; w[4 * i + 3] = r.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < KS; ++i) {
+                const uint2 r = __ldg(static_cast<const uint2 *>(p) + i);
+                w[2 * i] = r.x; w[2 * i + 1] = r.y;
             }
         }
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) acc[n][c] = 0.f;
-    };
-    flush();  // clears the accumulators
-#pragma unroll
-    for (int n = 0; n < 8; ++n) va[n] = make_uint4(0u, 0u, 0u, 0u);
+    }
+};
 
-    for (unsigned int sp = blockIdx.x * warps_per_block + warp; sp < nspan; sp += gridDim.x * warps_per_block) {
-        const unsigned int w0 = e_begin + sp * span;
-        const unsigned int wn = (e_end - w0 < span) ? e_end - w0 : span;  // entries of this warp's span
-        __syncwarp();  // the readers of the previous span are done with the records
-        for (unsigned int v = lane; v < 2 * wn; v += 32) {
-            const unsigned int sg = v / (2u * S);
-            ent_s[sg * seg_stride + (v - sg * 2u * S)] = __ldcs(p.sort_entries + 2 * (size_t)w0 + v);
+constexpr int kWalkSpan = 128;     // list entries a warp takes at a time
+constexpr int kWalkWarps = 4;
+constexpr int kWalkRegions = 160;  // most (level, head) regions of one launch
+struct WalkBuffer {                // per warp, double-buffered; padded so that a unit may be read past its end
+    float4 geo[kWalkSpan + 8];     // fractions along x, y, z, probability
+    uint4 tag[kWalkSpan + 8];      // row, (in a unit's first entry) end of the unit, base offset, corner mask
+};
+struct WalkShared {
+    WalkBuffer buf[kWalkWarps][2];
+    float4 dots[kWalkWarps][2][kWalkSpan];  // dot products of a point with corners 0-3 / 4-7
+};
+
+// The list of a (level, head) region is cut into spans, one warp each; a span into runs of points with the same cell, runs
+// into units of at most eight points; a warp takes two units at a time (halves A and B, one cell each).  With the eight
+// value rows V of the cell (one per corner), the grad_output rows GO of the unit's points and the points' corner weights
+// W, everything is small matrix products:
+//
+//   dot[point][corner]    = GO  V^T       m16n8k16: rows 0-7 the points of A, 8-15 of B; columns = corners of A's (B's) cell
+//   image[channel][corner] += GO^T W      m16n8k8 per half; W in three 16-bit terms (exact), GO^T by 8x8 transpositions
+//
+// Fragments come straight from 16-byte loads: lane (grp, tig) of a row-major fragment holds row grp's channels
+// tig*D/4 ..., for GO and V alike, so the order of the channels inside the product does not matter.  Rows of the next pair
+// of units travel while one is computed.  The image accumulators of a run stay in registers from unit to unit (4 * KS per
+// lane) and leave with full-line reductions when the run ends.  The dot products go to shared memory; after the span's
+// last unit a lane takes a point and turns its eight into the point's gradients.  All branches are uniform over the warp.
+//
+// 21 instructions per point on the largest pyramid (59 before, one lane group per point with 64 accumulators of its own and
+// the groups of a warp changing runs at different times), 33 at 4.5 points per run.  Bound by the L1 request pipe where the
+// volume fits L2 (76 % of its wavefronts: one per 64-byte row, two per reduction), by random 64-byte reads of grad_output
+// from DRAM on the largest: 4.7 M points 490 -> 263 us, 229.6 M points 19.3 -> 9.7 ms.
+//
+// A unit of fewer than eight points repeats its last point with weight zero (an infinite grad_output row then gives NaN
+// where a scalar sum gives infinity; both mark the same elements).
+template <typename VT, int KS>
+__global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 2)) fda_sorted_walk_kernel(const Problem p) {
+    static_assert(Vec16<VT>::kCPL == 8, "16-bit value dtypes only");
+    using Mma = WarpMma<VT>;
+    constexpr int kQuarter = 4 * KS;     // channels of a lane's part of a row
+    __shared__ LevelGeom geom[kMaxLevels];
+    __shared__ unsigned int region_entry[kWalkRegions + 1], region_span[kWalkRegions + 1];  // first entry / span of every region
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    WalkShared &sm = *reinterpret_cast<WalkShared *>(walk_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = blockIdx.y;
+    const int level_begin = __ffs(p.level_mask) - 1, level_end = 32 - __clz(p.level_mask);  // a contiguous range
+    const int regions = (level_end - level_begin) * p.G;
+    if (tid == 0) build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, true, p.l2_keep_bytes);
+    {
+        SortBins bins;
+        build_sort_bins(bins, p.shapes, p.L, p.G);
+        const unsigned int *starts = p.sort_counters + (size_t)b * bins.first[p.L];
+        for (int r = tid; r <= regions; r += blockDim.x) {
+            unsigned int bin = bins.first[level_end];
+            if (r < regions) {
+                const int l = level_begin + r / p.G;
+                bin = bins.first[l] + (unsigned int)(r % p.G) * bins.cells[l];
+            }
+            region_entry[r] = starts[bin];
         }
-        __syncwarp();
-        const unsigned int t0 = (unsigned int)grp * S;  // this group's segment inside the span
-        const unsigned int tn = t0 < wn ? (wn - t0 < S ? wn - t0 : S) : 0u;
-        const float4 *ent_g = ent_s + (unsigned int)grp * seg_stride;
-
-        // Asks for everything point t needs from global memory: its grad_output row, and -- when it starts a run, i.e.
-        // its cell or head differs from the previous point's or it is the first of the segment -- the eight value rows.
-        // Every lane commits one (possibly empty) copy group per point, so that "all but the newest kAhead - 1 groups
-        // are complete" always means "the rows of the current point have arrived".
-        auto request = [&](unsigned int t) {
-            if (t < tn) {
-                const float4 tag = ent_g[2 * t + 1];
-                uint4 *slot = ring + (size_t)((t % (unsigned int)kAhead) * kWalkSlot) * blockDim.x;
-                cp_async16_once(slot, go_base + (size_t)__float_as_uint(tag.x) * (size_t)p.D);
-                const unsigned int meta = __float_as_uint(tag.y), off0 = __float_as_uint(tag.z);
-                bool starts = t == 0;
-                if (!starts) {
-                    const float4 prev = ent_g[2 * t - 1];
-                    starts = __float_as_uint(prev.y) != meta || __float_as_uint(prev.z) != off0;
-                }
-                if (starts) {
-                    const LevelGeom lv = geom[meta & 15u];
-                    const uint32_t sx = (uint32_t)p.GD, sy = (uint32_t)lv.W * sx, sz = (uint32_t)lv.H * sy;
-                    const VT *lvl = value_b + (size_t)lv.start * p.GD + (size_t)((meta >> 4) & 0xffffu) * p.D;
-                    const unsigned int in8 = meta >> 20;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        unsigned int carry = 0;
+        for (int r0 = 0; r0 <= regions; r0 += 32) {  // uniform trip count
+            const int r = r0 + lane;
+            const unsigned int n = r < regions ? (region_entry[r + 1] - region_entry[r] + kWalkSpan - 1) / kWalkSpan : 0u;
+            unsigned int inc = n;
 #pragma unroll
-                    for (int n = 0; n < 8; ++n) {
-                        const bool in = (in8 >> n) & 1u;
-                        if (in) cp_async16(slot + (size_t)(1 + n) * blockDim.x,
-                                           lvl + (uint32_t)(off0 + ((n & 4) ? sz : 0u) + ((n & 2) ? sy : 0u) + ((n & 1) ? sx : 0u)));
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned int t = __shfl_up_sync(0xffffffffu, inc, d);
+                if (lane >= d) inc += t;
+            }
+            if (r <= regions) region_span[r] = carry + inc - n;
+            carry += __shfl_sync(0xffffffffu, inc, 31);
+        }
+    }
+    __syncthreads();
+    const unsigned int spans = region_span[regions];
+    const int tig = lane & 3, grp = lane >> 2;
+    const uint64_t pol_keep = l2_policy_evict_last(), pol_stream = l2_policy_evict_first();
+    const VT *go_base = static_cast<const VT *>(p.grad_out) + tig * kQuarter;
+    const bool odd = grp & 1;
+    // weight of corner grp along an axis = base + step * fraction
+    const float bx = (grp & 1) ? 0.f : 1.f, sx = (grp & 1) ? 1.f : -1.f;
+    const float by = (grp & 2) ? 0.f : 1.f, sy = (grp & 2) ? 1.f : -1.f;
+    const float bz = (grp & 4) ? 0.f : 1.f, sz = (grp & 4) ? 1.f : -1.f;
+    float4 (*dots)[kWalkSpan] = sm.dots[warp];
+
+    float carry[KS][4];  // image of the run that may go on
+    auto clear = [&]() {
+#pragma unroll
+        for (int k = 0; k < KS; ++k) { carry[k][0] = carry[k][1] = carry[k][2] = carry[k][3] = 0.f; }
+    };
+
+    auto request_span = [&](unsigned int sp, int r, int which) {  // copies a span's records; commits one (possibly empty) group
+        if (sp < spans) {
+            const unsigned int w0 = region_entry[r] + (sp - region_span[r]) * kWalkSpan;
+            const unsigned int left = region_entry[r + 1] - w0, wn = left < (unsigned int)kWalkSpan ? left : (unsigned int)kWalkSpan;
+            WalkBuffer &bf = sm.buf[warp][which];
+            const float4 *src = p.sort_entries + 2 * (size_t)w0;
+            void *dst = (lane & 1) ? static_cast<void *>(bf.tag) : static_cast<void *>(bf.geo);
+            for (unsigned int v = lane; v < 2 * wn; v += 32) cp_async16_once(static_cast<char *>(dst) + 16 * (v >> 1), src + v);
+        }
+        cp_async_commit();
+    };
+
+    const unsigned int stride = gridDim.x * kWalkWarps;
+    unsigned int sp = blockIdx.x * kWalkWarps + warp;
+    int region = 0, which = 0;
+    while (region < regions && sp >= region_span[region + 1]) ++region;
+    request_span(sp, region, 0);
+    for (; sp < spans; sp += stride, which ^= 1) {
+        int next_region = region;
+        while (next_region < regions && sp + stride >= region_span[next_region + 1]) ++next_region;
+        request_span(sp + stride, next_region, which ^ 1);
+        cp_async_wait<1>();
+        __syncwarp();
+        const unsigned int w0 = region_entry[region] + (sp - region_span[region]) * kWalkSpan;
+        const unsigned int left = region_entry[region + 1] - w0;
+        const int wn = (int)(left < (unsigned int)kWalkSpan ? left : (unsigned int)kWalkSpan);
+        const float4 *geo = sm.buf[warp][which].geo;
+        uint4 *tag = sm.buf[warp][which].tag;
+
+        // the region's level and head: uniform over the span
+        const int level = level_begin + region / p.G, head = region % p.G;
+        const LevelGeom lv = geom[level];
+        const uint32_t ox = (uint32_t)p.GD, oy = (uint32_t)lv.W * ox, oz = (uint32_t)lv.H * oy;
+        const size_t slice = (size_t)b * p.N * p.GD + (size_t)lv.start * p.GD + (size_t)head * p.D;
+        // value rows: corner grp, this lane's quarter of the channels
+        const VT *value_l = static_cast<const VT *>(p.value) + slice + tig * kQuarter;
+        const uint32_t corner = ((grp & 4) ? oz : 0u) + ((grp & 2) ? oy : 0u) + ((grp & 1) ? ox : 0u);
+        // image rows: corners 2 * tig and 2 * tig + 1, one half of quarter grp / 2
+        float *image_l = p.accum + slice + (grp >> 1) * kQuarter + (grp & 1) * (2 * KS);
+        const uint32_t corner0 = ((tig & 2) ? oz : 0u) + ((tig & 1) ? oy : 0u);
+        const uint64_t pol_image = (lv.keep & 2) ? pol_keep : pol_stream;
+
+        // Sends a run's image.  carry[k][e]: word 2k + e/2 of quarter grp/2, i.e. channels 2 * word + odd, at corner
+        // 2 * tig + e%2.  Neighbouring lane groups hold the even and the odd channels; they swap so that each has a
+        // contiguous half.
+        auto flush = [&](uint32_t off0, unsigned int in8) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float out[2 * KS];
+#pragma unroll
+                for (int j = 0; j < KS; ++j) {   // words j (first half) and KS + j (second half) of the quarter
+                    const float first = carry[j >> 1][2 * (j & 1) + e], second = carry[(KS + j) >> 1][2 * ((KS + j) & 1) + e];
+                    const float mine = odd ? second : first;
+                    const float other = __shfl_xor_sync(0xffffffffu, odd ? first : second, 4);
+                    out[2 * j] = (odd ? other : mine) * Mma::kUnscale;
+                    out[2 * j + 1] = (odd ? mine : other) * Mma::kUnscale;
+                }
+                if (in8 >> (2 * tig + e) & 1u) {
+                    float *dst = image_l + (uint32_t)(off0 + corner0 + (e ? ox : 0u));
+                    if constexpr (KS % 2 == 0) {
+#pragma unroll
+                        for (int i = 0; i < KS / 2; ++i) red_add_f32x4_hint(dst + 4 * i, out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3], pol_image);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < KS; ++i) red_add_f32x2_hint(dst + 2 * i, out[2 * i], out[2 * i + 1], pol_image);
                     }
                 }
             }
-            cp_async_commit();
+            clear();
         };
-        for (unsigned int k = 0; k < (unsigned int)kAhead; ++k) request(k);
-        for (unsigned int t = 0; t < S; ++t) {  // uniform trip count: the matrix instructions need the whole warp
-            const bool have = t < tn;
-            float4 ent = make_float4(0.f, 0.f, 0.f, 0.f), tag = ent;
-            if (have) {
-                ent = ent_g[2 * t];       // voxel x, y, z, probability
-                tag = ent_g[2 * t + 1];   // row, level | head << 4 | corner mask << 20, base offset, point index inside the row
+
+        // units: an entry starts one when it is the 1st, 9th, 17th ... of its run; it is told where its unit ends
+        unsigned int unit_mask[kWalkSpan / 32];
+        int run_start = 0;
+#pragma unroll
+        for (int g = 0; g < kWalkSpan / 32; ++g) {
+            const int e = g * 32 + lane;
+            const bool ok = e < wn;
+            bool starts = e == 0;
+            if (ok && !starts) {
+                const uint2 t = *reinterpret_cast<const uint2 *>(&tag[e].z), q = *reinterpret_cast<const uint2 *>(&tag[e - 1].z);
+                starts = q.x != t.x || q.y != t.y;
             }
-            const unsigned int meta = __float_as_uint(tag.y), off0 = __float_as_uint(tag.z);
-            cp_async_wait<kAhead - 1>();
-            const uint4 *slot = ring + (size_t)((t % (unsigned int)kAhead) * kWalkSlot) * blockDim.x;
-            if (have && (meta != run_meta || off0 != run_off)) {
-                flush();
-                run_meta = meta;
-                run_off = off0;
-                const unsigned int in8 = meta >> 20;
-#pragma unroll
-                for (int n = 0; n < 8; ++n) {
-                    const bool in = (in8 >> n) & 1u;
-                    va[n] = in ? slot[(size_t)(1 + n) * blockDim.x] : make_uint4(0u, 0u, 0u, 0u);
-                }
-            }
-            uint4 gr = make_uint4(0u, 0u, 0u, 0u);
-            if (have) gr = slot[0];
-            // the weights of point_geometry_voxel
-            const float xf = floorf(ent.x), yf = floorf(ent.y), zf = floorf(ent.z);
-            const float wx[2] = {__fsub_rn(__fadd_rn(xf, 1.0f), ent.x), __fsub_rn(ent.x, xf)};
-            const float wy[2] = {__fsub_rn(__fadd_rn(yf, 1.0f), ent.y), __fsub_rn(ent.y, yf)};
-            const float wz[2] = {__fsub_rn(__fadd_rn(zf, 1.0f), ent.z), __fsub_rn(ent.z, zf)};
-            const float a = have ? ent.w : 0.f;
-            float dot[8];
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                float c[4];
-                // a group without a point in this iteration multiplies stale rows with a zero grad_output row
-                MmaDot<VT>::first(c, va[2 * h].x, va[2 * h + 1].x, va[2 * h].y, va[2 * h + 1].y, gr.x, gr.y);
-                MmaDot<VT>::mma(c, va[2 * h].z, va[2 * h + 1].z, va[2 * h].w, va[2 * h + 1].w, gr.z, gr.w);
-                dot[2 * h] = odd ? c[1] : c[0];  // meaningful in the owner lane only
-                dot[2 * h + 1] = odd ? c[3] : c[2];
-            }
-            // Every lane does the owner's arithmetic (the warp pays for it either way): the corner weights are then
-            // shared between the point's own gradients and its contribution to the image rows.
-            const float wyx[4] = {wy[0] * wx[0], wy[0] * wx[1], wy[1] * wx[0], wy[1] * wx[1]};
-            const float wzy[4] = {wz[0] * wy[0], wz[0] * wy[1], wz[1] * wy[0], wz[1] * wy[1]};
-            const float wzx[4] = {wz[0] * wx[0], wz[0] * wx[1], wz[1] * wx[0], wz[1] * wx[1]};
-            float w[8];  // corner n = dz*4 + dy*2 + dx
-#pragma unroll
-            for (int n = 0; n < 8; ++n) w[n] = wyx[n & 3] * wz[n >> 2];
-            const float gx = wzy[0] * (dot[1] - dot[0]) + wzy[1] * (dot[3] - dot[2]) + wzy[2] * (dot[5] - dot[4]) + wzy[3] * (dot[7] - dot[6]);
-            const float gy = wzx[0] * (dot[2] - dot[0]) + wzx[1] * (dot[3] - dot[1]) + wzx[2] * (dot[6] - dot[4]) + wzx[3] * (dot[7] - dot[5]);
-            const float gz = wyx[0] * (dot[4] - dot[0]) + wyx[1] * (dot[5] - dot[1]) + wyx[2] * (dot[6] - dot[2]) + wyx[3] * (dot[7] - dot[3]);
-            float da = 0.f;
-#pragma unroll
-            for (int n = 0; n < 8; ++n) da = fmaf(w[n], dot[n], da);
-            if (have && tig == owner) {
-                const LevelGeom lv = geom[meta & 15u];
-                __stcs(p.sort_results + (size_t)__float_as_uint(tag.x) * (size_t)p.LK + __float_as_uint(tag.w),
-                       make_float4(a * lv.fW * gx, a * lv.fH * gy, a * lv.fD * gz, da));
-            }
-            float god[8];
-            Vec16<VT>::unpack(gr, god);
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                // corners outside the level collect finite garbage that flush() never sends (same run, same corners)
-                const float aw = a * w[n];
-#pragma unroll
-                for (int c = 0; c < 8; c += 2) ffma2(acc[n][c], acc[n][c + 1], aw, aw, god[c], god[c + 1]);
-            }
-            request(t + kAhead);  // into the slot just read
+            const unsigned int run_mask = __ballot_sync(0xffffffffu, starts);
+            const unsigned int upto = run_mask & (0xffffffffu >> (31 - lane));
+            const int mine = upto ? g * 32 + 31 - __clz(upto) : run_start;
+            if (run_mask) run_start = g * 32 + 31 - __clz(run_mask);
+            unit_mask[g] = __ballot_sync(0xffffffffu, ok && ((e - mine) & 7) == 0);
         }
-        cp_async_wait<0>();
-        flush();
-        run_meta = kNoRun;
+        int next_first = wn;
+#pragma unroll
+        for (int g = kWalkSpan / 32 - 1; g >= 0; --g) {
+            const unsigned int later = unit_mask[g] & ~(0xffffffffu >> (31 - lane));
+            if (unit_mask[g] >> lane & 1u) tag[g * 32 + lane].y = (unsigned int)(later ? g * 32 + __ffs(later) - 1 : next_first);
+            if (unit_mask[g]) next_first = g * 32 + __ffs(unit_mask[g]) - 1;
+        }
+        if (lane == 0) {  // an empty unit behind the last one goes on with its run: half B of an odd last pair
+            const uint4 t = tag[wn - 1];
+            tag[wn] = make_uint4(t.x, (unsigned int)wn, t.z, t.w);
+        }
+        __syncwarp();
+
+        struct Half {
+            RowWords<KS> go, v;
+            int first, last;
+            uint2 run;  // base offset, corner mask
+            __device__ __forceinline__ bool same(const uint2 &o) const { return run.x == o.x && run.y == o.y; }
+        };
+        auto request = [&](Half &h, int first) {  // asks for the rows of the unit that starts at entry `first`
+            const uint4 t = tag[first];
+            h.first = first;
+            h.last = (int)t.y;
+            h.run = make_uint2(t.z, t.w);
+            const int at = min(first + grp, max(h.last - 1, 0));
+            h.go.load(go_base + (size_t)tag[at].x * (size_t)p.D);
+            h.v.zero();
+            if (t.w >> grp & 1u) h.v.load(value_l + (uint32_t)(t.z + corner));
+        };
+        // image += GO^T W of a unit, into fresh accumulators (no product waits for another unit's)
+        auto scatter = [&](const Half &h, float (&acc)[KS][4]) {
+            float w[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int i = h.first + 2 * tig + e;
+                const float4 g = geo[i];
+                const float wp = (g.w * Mma::kScale) * ((fmaf(sx, g.x, bx) * fmaf(sy, g.y, by)) * fmaf(sz, g.z, bz));
+                w[e] = i < h.last ? wp : 0.f;
+            }
+            uint32_t got[2 * KS];
+#pragma unroll
+            for (int i = 0; i < 2 * KS; ++i) got[i] = transpose8x8(h.go.w[i]);
+#pragma unroll
+            for (int k = 0; k < KS; ++k) { acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.f; }
+#pragma unroll
+            for (int term = 0; term < 3; ++term) {
+                const uint32_t wt = Mma::take(w[0], w[1]);
+#pragma unroll
+                for (int k = 0; k < KS; ++k) Mma::k8(acc[k], got[2 * k], got[2 * k + 1], wt);
+            }
+        };
+        auto add = [&](const float (&acc)[KS][4]) {
+#pragma unroll
+            for (int k = 0; k < KS; ++k)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) carry[k][e] += acc[k][e];
+        };
+        uint2 run = make_uint2(0u, 0u);  // no run yet: no corner, nothing is sent
+        auto pair = [&](const Half &ha, const Half &hb) {
+            float ca[4] = {0.f, 0.f, 0.f, 0.f}, cb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int k = 0; k < KS; ++k) {
+                Mma::k16(ca, ha.go.w[2 * k], hb.go.w[2 * k], ha.go.w[2 * k + 1], hb.go.w[2 * k + 1], ha.v.w[2 * k], ha.v.w[2 * k + 1]);
+                Mma::k16(cb, ha.go.w[2 * k], hb.go.w[2 * k], ha.go.w[2 * k + 1], hb.go.w[2 * k + 1], hb.v.w[2 * k], hb.v.w[2 * k + 1]);
+            }
+            float ia[KS][4], ib[KS][4];
+            scatter(ha, ia);
+            scatter(hb, ib);
+            // corners 2 * tig and 2 * tig + 1 of point grp
+            const int pa = ha.first + grp, pb = hb.first + grp;
+            if (pa < ha.last) *(reinterpret_cast<float2 *>(&dots[tig >> 1][pa]) + (tig & 1)) = make_float2(ca[0], ca[1]);
+            if (pb < hb.last) *(reinterpret_cast<float2 *>(&dots[tig >> 1][pb]) + (tig & 1)) = make_float2(cb[2], cb[3]);
+            if (!ha.same(run)) flush(run.x, run.y);
+            add(ia);
+            if (!hb.same(ha.run)) flush(ha.run.x, ha.run.y);
+            add(ib);
+            run = hb.run;
+        };
+        clear();
+        Half h0, h1, h2, h3;
+        request(h0, 0);
+        request(h1, h0.last);
+        for (;;) {  // two pairs per turn: the register sets alternate without copies
+            bool more = h1.last < wn;
+            if (more) {
+                request(h2, h1.last);
+                request(h3, h2.last);
+            }
+            pair(h0, h1);
+            if (!more) break;
+            more = h3.last < wn;
+            if (more) {
+                request(h0, h3.last);
+                request(h1, h0.last);
+            }
+            pair(h2, h3);
+            if (!more) break;
+        }
+        flush(run.x, run.y);
+        __syncwarp();
+
+        // the points' own gradients, one point per lane
+        for (int e = lane; e < wn; e += 32) {
+            const float4 lo = dots[0][e], hi = dots[1][e], g = geo[e];
+            const float x0 = 1.0f - g.x, y0 = 1.0f - g.y, z0 = 1.0f - g.z;
+            // along x: interpolated value s and difference d for (z, y) = 00, 01, 10, 11
+            const float s00 = fmaf(g.x, lo.y, x0 * lo.x), s01 = fmaf(g.x, lo.w, x0 * lo.z), d00 = lo.y - lo.x, d01 = lo.w - lo.z;
+            const float s10 = fmaf(g.x, hi.y, x0 * hi.x), s11 = fmaf(g.x, hi.w, x0 * hi.z), d10 = hi.y - hi.x, d11 = hi.w - hi.z;
+            // along y
+            const float s0 = fmaf(g.y, s01, y0 * s00), s1 = fmaf(g.y, s11, y0 * s10);
+            const float dx0 = fmaf(g.y, d01, y0 * d00), dx1 = fmaf(g.y, d11, y0 * d10);
+            const float gx = fmaf(g.z, dx1, z0 * dx0), gy = fmaf(g.z, s11 - s10, z0 * (s01 - s00)), gz = s1 - s0, da = fmaf(g.z, s1, z0 * s0);
+            __stcs(p.sort_results + w0 + e, make_float4(g.w * lv.fW * gx, g.w * lv.fH * gy, g.w * lv.fD * gz, da));
+        }
+        __syncwarp();  // records, units and dot products have been read
+        region = next_region;
     }
+    cp_async_wait<0>();
 }
 
-// Per row: the results of its points, soft-max backward, finished row of grad_sampling_loc_attn.  A point without a
-// corner inside its level was never filed and has no result: its gradients are zero (the same test as in the fill pass).
+// Per row: the results of its points from the list, soft-max backward grad_logit_i = p_i * (dalpha_i - sum_j p_j dalpha_j),
+// finished row of grad_sampling_loc_attn.  A point that is not filed has no result: its gradients are zero.  One random
+// 16-byte read per point; scattered 16-byte writes in the walk instead cost as much when the results fit L2 and three times
+// the DRAM traffic when they do not.
 template <typename PT>
 __global__ void __launch_bounds__(kThreads) fda_sort_finalize_kernel(const Problem p) {
-    __shared__ LevelGeom geom[kMaxLevels];
     extern __shared__ __align__(16) float smem_tile[];
-    const int tid = threadIdx.x;
-    if (tid == 0) build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, false, 0ull);
-    const int b = blockIdx.y;
+    const int tid = threadIdx.x, b = blockIdx.y;
     const int gs = 1 << p.gs_log2;
     const int lane = tid & 31, warp = tid >> 5;
     const int lane_c = tid & (gs - 1);
@@ -480,63 +713,46 @@ __global__ void __launch_bounds__(kThreads) fda_sort_finalize_kernel(const Probl
     float *wtile = smem_tile + warp * rows_per_warp * p.row_stride;
     int nrows = p.rows_per_b - first;
     nrows = nrows < 0 ? 0 : (nrows > rows_per_warp ? rows_per_warp : nrows);
-    const size_t warp_elem0 = ((size_t)b * p.rows_per_b + first) * (size_t)(4 * LK);
-    stage_rows<PT>(static_cast<const PT *>(p.packed) + warp_elem0, wtile, nrows, LK, p.row_stride, lane);
-    __syncthreads();  // level table and this warp's tile visible
     float *trow = wtile + (lane >> p.gs_log2) * p.row_stride;
     const size_t rowg = (size_t)b * p.rows_per_b + (row_ok ? row : 0);
-    const unsigned int g = row_ok ? (unsigned int)(row % p.G) : 0u;
-    const float4 *results = p.sort_results + rowg * (size_t)LK;
-    const int rounds = (LK + gs - 1) >> p.gs_log2;  // uniform over the warp
+    const unsigned int *positions = p.sort_ranks + rowg * (size_t)LK;
+    const PT *logits = static_cast<const PT *>(p.packed) + rowg * (size_t)(4 * LK) + 3 * LK;
+    const float2 stats = __ldg(p.sort_stats + rowg);
 
-    // Tile row layout: [0,3LK) coordinates -> coordinate gradients, [3LK,4LK) logits -> dalpha -> logit gradients,
-    // [4LK,5LK) exp(logit - max).
-    float m = -INFINITY;
-    for (int j = 0; j < rounds; ++j) {
-        const int i = lane_c + j * gs;
-        if (row_ok && i < LK) m = fmaxf(m, trow[3 * LK + i]);
-    }
-    for (int mask = gs >> 1; mask > 0; mask >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, mask));
-    float s = 0.f, S = 0.f;
+    // Tile row: [0,3LK) coordinate gradients, [3LK,4LK) dalpha -> logit gradients, [4LK,5LK) probabilities.
+    float S = 0.f;
     constexpr int kBatch = 8;  // the results of eight points are requested before the first one is used
-    for (int j0 = 0; j0 < rounds; j0 += kBatch) {
+    for (int i0 = lane_c; row_ok && i0 < LK; i0 += kBatch * gs) {
+        unsigned int at[kBatch];
+        float lg[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int i = i0 + u * gs;
+            at[u] = i < LK ? __ldcs(positions + i) : kNoPosition;
+            lg[u] = i < LK ? load1<PT>(logits + i) : 0.f;
+        }
         float4 r[kBatch];
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-            const int i = lane_c + (j0 + j) * gs;
-            r[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row_ok && i < LK) {
-                const LevelGeom lv = geom[(i >> 2) >> p.k_shift];
-                const SortTag tag = sort_tag_of(lv, p.G, p.GD, g, unnormalize(trow[3 * i], lv.fW), unnormalize(trow[3 * i + 1], lv.fH),
-                                                unnormalize(trow[3 * i + 2], lv.fD));
-                if (tag.ok) r[j] = __ldcs(results + i);
-            }
+        for (int u = 0; u < kBatch; ++u) {
+            r[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (at[u] != kNoPosition) r[u] = __ldcs(p.sort_results + at[u]);
         }
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-            const int i = lane_c + (j0 + j) * gs;
-            if (row_ok && i < LK) {
-                const float ex = __expf(trow[3 * LK + i] - m);
-                trow[3 * i] = r[j].x; trow[3 * i + 1] = r[j].y; trow[3 * i + 2] = r[j].z;
-                trow[3 * LK + i] = r[j].w;   // dalpha
-                trow[4 * LK + i] = ex;
-                s += ex;
-                S = fmaf(ex, r[j].w, S);
+        for (int u = 0; u < kBatch; ++u) {
+            const int i = i0 + u * gs;
+            if (i < LK) {
+                const float a = __expf(lg[u] - stats.x) * stats.y;
+                trow[3 * i] = r[u].x; trow[3 * i + 1] = r[u].y; trow[3 * i + 2] = r[u].z;
+                trow[3 * LK + i] = r[u].w;
+                trow[4 * LK + i] = a;
+                S = fmaf(a, r[u].w, S);
             }
         }
     }
-    for (int mask = gs >> 1; mask > 0; mask >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, mask);
-        S += __shfl_xor_sync(0xffffffffu, S, mask);
-    }
-    const float inv = row_ok ? 1.0f / s : 0.f;
-    S *= inv;  // sum_i p_i * dalpha_i
-    for (int j = 0; j < rounds; ++j) {
-        const int i = lane_c + j * gs;
-        if (row_ok && i < LK) trow[3 * LK + i] = trow[4 * LK + i] * inv * (trow[3 * LK + i] - S);
-    }
+    for (int mask = gs >> 1; mask > 0; mask >>= 1) S += __shfl_xor_sync(0xffffffffu, S, mask);
+    for (int i = lane_c; row_ok && i < LK; i += gs) trow[3 * LK + i] = trow[4 * LK + i] * (trow[3 * LK + i] - S);
     __syncwarp();
-    PT *dst = static_cast<PT *>(p.grad_packed) + warp_elem0;
+    PT *dst = static_cast<PT *>(p.grad_packed) + ((size_t)b * p.rows_per_b + first) * (size_t)(4 * LK);
     const int nvec = nrows * LK;
     const float inv_lk = 1.0f / (float)LK;
     for (int v = lane; v < nvec; v += 32) {

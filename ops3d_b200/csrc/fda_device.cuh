@@ -71,13 +71,14 @@ struct Problem {
     // level range); null: the logit slots of grad_packed carry it (exact only when the packed dtype is fp32)
     float *dalpha;
     // backward, cell-sorted handling of all levels (see fda_backward_sorted.cuh); null: not used
-    unsigned int *sort_counters;   // [B*N*G]: points per (batch, cell, head) -> exclusive scan -> end of each bin
+    unsigned int *sort_counters;   // per (batch, level, head, base cell): points -> exclusive scan; then the length of the list
     unsigned int *sort_tile_sums;  // scratch of the scan
-    float4 *sort_entries;          // sorted list, 32 bytes per point: {voxel x, y, z inside the point's level, soft-max
-                                   // probability} {row b*Q*G + q*G + g, level | head << 4 | corner mask << 20, element
-                                   // offset of the base corner, index of the point inside its row}
-    float4 *sort_results;          // [B*Q*G][L*K] in row order: {d/dx, d/dy, d/dz, dalpha} of every filed point
-    int sort_seg;                  // list entries one lane group walks before it flushes its accumulators
+    float2 *sort_stats;            // [B*Q*G]: soft-max statistics {max, 1 / sum} of every row
+    unsigned int *sort_ranks;      // [B*Q*G][L*K]: rank of a point inside its bin -> its position in the list
+    float4 *sort_entries;          // sorted list, 32 bytes per point: {fractions of the voxel position along x, y, z,
+                                   // soft-max probability} {row b*Q*G + q*G + g, unused, element offset of the base corner,
+                                   // corner mask}
+    float4 *sort_results;          // {d/dx, d/dy, d/dz, dalpha} of every filed point, in list order
 };
 
 constexpr int kMaxSlabs = 128;
@@ -345,6 +346,9 @@ template <> __device__ __forceinline__ float4 cvt4<__half>(const uint4 &r) {
 __device__ __forceinline__ void red_add_f32x4_hint(float *p, float a, float b, float c, float d, uint64_t pol) {
     asm volatile("red.global.add.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;"
                  ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void red_add_f32x2_hint(float *p, float a, float b, uint64_t pol) {
+    asm volatile("red.global.add.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(a), "f"(b), "l"(pol) : "memory");
 }
 __device__ __forceinline__ void stg16_hint(void *p, const uint4 &v, uint64_t pol) {
     asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;"

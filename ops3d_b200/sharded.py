@@ -273,7 +273,7 @@ class PeerReducer:
         slab = None
         # the cell-sorted backward (when the library chooses it for this rank's rows) works level range by level range,
         # not slab group by slab group
-        sorted_path = capi.backward_path(value[:1], packed[:1], K) == 2
+        sorted_path = capi.backward_path(value[:1], packed[:1], K) >= 2
         if passes is not None and nbytes and not sorted_path:
             plan = capi.bin_plan(self.shapes_host, one, packed.shape[1], K)
             if plan is not None:

@@ -362,7 +362,8 @@ int fda_pack_sampling_backward(const float *grad_packed, const int64_t *spatial_
  * csrc/dcnv4.h:7-61).  d_stride / block_thread of the reference are launch hints and have no counterpart here.
  * The backward zero-fills what it accumulates into and writes both gradients completely (offset-row padding = 0);
  * gradients come back in the tensors' own dtype.  workspace: fda_dcnv4_backward_workspace_bytes() (an fp32 image of
- * grad_value for 16-bit dtypes, none for fp32), 16-byte aligned.
+ * grad_value for 16-bit dtypes, none for fp32), 16-byte aligned.  With fda_dcnv4_backward_scratch_bytes() (at least as
+ * much; 256-byte aligned) large 16-bit problems take the cell-sorted path; with less the call takes the plain one.
  */
 int fda_dcnv4_output_size(int depth_in, int height_in, int width_in, const int *kernel, const int *stride,
                           const int *pad, const int *dilation, int *depth_out, int *height_out, int *width_out);
@@ -372,6 +373,9 @@ int fda_dcnv4_forward(const void *value, const void *p_offset, void *output, int
                       int padded_offset_dim, int dtype, int im2col_step, void *stream);
 size_t fda_dcnv4_backward_workspace_bytes(int batch, int depth_in, int height_in, int width_in, int group,
                                           int group_channels, int dtype);
+size_t fda_dcnv4_backward_scratch_bytes(int batch, int depth_in, int height_in, int width_in, int group,
+                                        int group_channels, const int *kernel, const int *stride, const int *pad,
+                                        const int *dilation, int remove_center, int softmax, int dtype);
 int fda_dcnv4_backward(const void *value, const void *p_offset, const void *grad_output, void *grad_value,
                        void *grad_offset, void *workspace, size_t workspace_bytes, int batch, int depth_in,
                        int height_in, int width_in, int group, int group_channels, const int *kernel,

@@ -20,7 +20,7 @@ EXPORTS = (
     "fda_backward_noalloc", "fda_peer_reduce_cast", "fda_multimem_reduce_cast", "fda_backward_accumulate_levels",
     "fda_peer_push_partials", "fda_peer_reduce_staged_cast", "fda_backward_bin_plan", "fda_backward_binned_part",
     "fda_pack_sampling", "fda_pack_sampling_backward", "fda_dcnv4_forward", "fda_dcnv4_backward",
-    "fda_dcnv4_backward_workspace_bytes", "fda_dcnv4_output_size", "fda_roi_align3d_forward", "fda_roi_align3d_backward",
+    "fda_dcnv4_backward_workspace_bytes", "fda_dcnv4_backward_scratch_bytes", "fda_dcnv4_output_size", "fda_roi_align3d_forward", "fda_roi_align3d_backward",
     "fda_nms3d", "fda_nms3d_workspace_bytes", "fda_nms3d_scored", "fda_nms3d_scored_workspace_bytes", "fda_reload_config", "fda_group_reduce_cast", "fda_head_slice_cast_push",
     "fda_backward_touched_rows", "fda_cast_grad_value_touched",
 )
@@ -100,6 +100,8 @@ def load() -> ctypes.CDLL:
     lib.fda_dcnv4_forward.restype = i
     lib.fda_dcnv4_backward_workspace_bytes.argtypes = [i] * 7
     lib.fda_dcnv4_backward_workspace_bytes.restype = sz
+    lib.fda_dcnv4_backward_scratch_bytes.argtypes = [i] * 6 + [vp] * 4 + [i] * 3
+    lib.fda_dcnv4_backward_scratch_bytes.restype = sz
     lib.fda_dcnv4_backward.argtypes = [vp] * 6 + [sz] + [i] * 6 + [vp] * 4 + [f] + [i] * 5 + [vp]
     lib.fda_dcnv4_backward.restype = i
     lib.fda_roi_align3d_forward.argtypes = [vp] * 3 + [i] * 8 + [f] + [i] * 3 + [vp]
@@ -463,7 +465,9 @@ def dcnv4_backward(value, p_offset, grad_output, kernel, stride, pad, dilation, 
     """``fda_dcnv4_backward`` -> ``(grad_value, grad_offset)`` in the inputs' dtype."""
     B, Din, Hin, Win, C = value.shape
     grad_value, grad_offset = torch.empty_like(value), torch.empty_like(p_offset)
-    need = int(load().fda_dcnv4_backward_workspace_bytes(B, Din, Hin, Win, group, group_channels, DTYPE_CODE[value.dtype]))
+    need = int(load().fda_dcnv4_backward_scratch_bytes(B, Din, Hin, Win, group, group_channels, _triple(kernel), _triple(stride),
+                                                       _triple(pad), _triple(dilation), int(remove_center), int(bool(softmax)),
+                                                       DTYPE_CODE[value.dtype]))
     ws = torch.empty((need + 3) // 4, dtype=torch.float32, device=value.device) if need else None
     with torch.cuda.device(value.device):
         check(load().fda_dcnv4_backward(value.data_ptr(), p_offset.data_ptr(), grad_output.data_ptr(), grad_value.data_ptr(),

@@ -229,7 +229,8 @@ std::vector<at::Tensor> dcnv4_backward(const at::Tensor &value, const at::Tensor
     c10::cuda::CUDAGuard guard(value.device());
     at::Tensor grad_value = empty_as(value);
     at::Tensor grad_offset = empty_as(p_offset);
-    const size_t ws_bytes = fda_dcnv4_backward_workspace_bytes(d.B, d.Din, d.Hin, d.Win, group, group_channels, vdt);
+    const size_t ws_bytes = fda_dcnv4_backward_scratch_bytes(d.B, d.Din, d.Hin, d.Win, group, group_channels, kernel, stride, pad,
+                                                             dilation, remove_center, softmax ? 1 : 0, vdt);
     at::Tensor workspace;
     void *ws_ptr = nullptr;
     if (ws_bytes > 0) {

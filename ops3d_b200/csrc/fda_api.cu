@@ -270,7 +270,7 @@ SortLayout sort_layout(int B, int N, int G, int D, int L, int Q, int K, int vdt)
     const unsigned long long points = (unsigned long long)B * Q * G * L * K, rows = (unsigned long long)B * Q * G;
     if (bins >= (1ull << 31) || points >= (1ull << 31)) return s;
     if (g_config.sorted == 1 && !sorted_pays(D, (double)points, (double)Q * L * K / N)) return s;
-    s.tiles = (unsigned int)((bins + fda::kScanTile - 1) / fda::kScanTile);
+    s.tiles = fda::sort_scan_tiles(bins);
     s.counters = 0;
     s.tile_sums = round256(bins * sizeof(unsigned int));
     s.stats = s.tile_sums + round256((size_t)s.tiles * sizeof(unsigned int));
@@ -383,6 +383,30 @@ int launch_binned_part(fda::Problem p, cudaStream_t st) {
     return launch_binned_slabs<VT, PT>(p, st);
 }
 
+// Exclusive scan of the counters of `bins` bins (an upper bound; the kernels find the real number).
+int launch_scan(const fda::Problem &p, unsigned long long bins, cudaStream_t st) {
+    const unsigned int tiles = fda::sort_scan_tiles(bins);
+    fda::fda_scan_tile_sums_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p);
+    fda::fda_scan_spine_kernel<<<1, fda::kScanThreads, 0, st>>>(p);
+    fda::fda_scan_apply_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? FDA_OK : cuda_fail(e);
+}
+
+template <typename VT>
+int launch_walk(const fda::Problem &p, cudaStream_t st) {
+    auto walk = p.D == 16 ? fda::fda_sorted_walk_kernel<VT, 1> : (p.D == 32 ? fda::fda_sorted_walk_kernel<VT, 2>
+                : (p.D == 48 ? fda::fda_sorted_walk_kernel<VT, 3> : fda::fda_sorted_walk_kernel<VT, 4>));
+    const size_t walk_smem = sizeof(fda::WalkShared);
+    if (int rc = ensure_smem(reinterpret_cast<const void *>(walk), walk_smem)) return rc;
+    const int per_sm = p.D <= 32 ? 4 : (p.D == 48 ? 3 : 2);  // resident blocks, by registers
+    int gx = g_config.sort_grid_x;
+    if (gx <= 0) gx = (per_sm * sm_count() + p.B - 1) / p.B;
+    walk<<<dim3((unsigned)gx, (unsigned)p.B, 1), fda::kWalkWarps * 32, walk_smem, st>>>(p);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? FDA_OK : cuda_fail(e);
+}
+
 // Cell-sorted path: the first launch of a sequence sorts the points of ALL levels; every launch walks the part of
 // the list that belongs to its levels; the last one writes grad_sampling_loc_attn.
 template <typename VT, typename PT>
@@ -392,7 +416,6 @@ int launch_sorted(fda::Problem p, cudaStream_t st) {
     } else {
         if (!p.resume) {
             const unsigned long long bins = 8ull * p.B * p.N * p.G + 1;
-            const unsigned int tiles = (unsigned int)((bins + fda::kScanTile - 1) / fda::kScanTile);
             const unsigned long long clear_blocks = (bins + 1023) / 1024;
             fda::fda_sort_clear_kernel<<<(unsigned)(clear_blocks > 2368 ? 2368 : clear_blocks), 256, 0, st>>>(p);
             fda::Problem q = p;
@@ -402,23 +425,14 @@ int launch_sorted(fda::Problem p, cudaStream_t st) {
             auto count = fda::fda_sort_count_kernel<PT>;
             if (int rc = ensure_smem(reinterpret_cast<const void *>(count), smem)) return rc;
             count<<<row_grid(q, threads), threads, smem, st>>>(q);
-            fda::fda_scan_tile_sums_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p);
-            fda::fda_scan_spine_kernel<<<1, fda::kScanThreads, 0, st>>>(p);
-            fda::fda_scan_apply_kernel<<<tiles, fda::kScanThreads, 0, st>>>(p);
+            if (int rc = launch_scan(p, bins, st)) return rc;
             auto fill = fda::fda_sort_fill_kernel<PT>;
             if (int rc = ensure_smem(reinterpret_cast<const void *>(fill), smem)) return rc;
             fill<<<row_grid(q, threads), threads, smem, st>>>(q);
             const cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return cuda_fail(e);
         }
-        auto walk = p.D == 16 ? fda::fda_sorted_walk_kernel<VT, 1> : (p.D == 32 ? fda::fda_sorted_walk_kernel<VT, 2>
-                    : (p.D == 48 ? fda::fda_sorted_walk_kernel<VT, 3> : fda::fda_sorted_walk_kernel<VT, 4>));
-        const size_t walk_smem = sizeof(fda::WalkShared);
-        if (int rc = ensure_smem(reinterpret_cast<const void *>(walk), walk_smem)) return rc;
-        const int per_sm = p.D <= 32 ? 4 : (p.D == 48 ? 3 : 2);  // resident blocks, by registers
-        int gx = g_config.sort_grid_x;
-        if (gx <= 0) gx = (per_sm * sm_count() + p.B - 1) / p.B;
-        walk<<<dim3((unsigned)gx, (unsigned)p.B, 1), fda::kWalkWarps * 32, walk_smem, st>>>(p);
+        if (int rc = launch_walk<VT>(p, st)) return rc;
         if (p.finalize) {
             fda::Problem q = p;
             q.row_stride = padded_stride(5 * p.LK);
@@ -491,6 +505,13 @@ int launch_backward(fda::Problem p, cudaStream_t st) {
 namespace fda {
 const Config &config() { return g_config; }
 void record_cuda_error(int e) { g_last_cuda_error = e; }
+unsigned int sort_scan_tiles(unsigned long long bins) { return (unsigned int)((bins + kScanTile - 1) / kScanTile); }
+int launch_sort_scan(const Problem &p, unsigned long long bins, cudaStream_t st) { return launch_scan(p, bins, st); }
+int launch_sort_walk(const Problem &p, int value_dtype, cudaStream_t st) {
+    if (value_dtype == FDA_DTYPE_F16) return launch_walk<__half>(p, st);
+    if (value_dtype == FDA_DTYPE_BF16) return launch_walk<__nv_bfloat16>(p, st);
+    return FDA_ERR_BAD_DTYPE;
+}
 }  // namespace fda
 
 extern "C" {

@@ -27,6 +27,7 @@
 #pragma once
 
 #include "fda_backward.cuh"
+#include "fda_sort_record.cuh"
 
 namespace fda {
 
@@ -67,12 +68,6 @@ __device__ __forceinline__ BaseCell base_cell(const LevelGeom &lv, float x, floa
 }
 __device__ __forceinline__ unsigned int bin_of(const LevelGeom &lv, const BaseCell &c) {  // inside its level and head
     return ((unsigned int)(c.z + 1) * (unsigned int)(lv.H + 1) + (unsigned int)(c.y + 1)) * (unsigned int)(lv.W + 1) + (unsigned int)(c.x + 1);
-}
-
-// One 32-byte list record as ONE streaming store (sm_100: 256-bit vector store); `rec` is 32-byte aligned.
-__device__ __forceinline__ void store_record(float4 *rec, const float4 &a, const float4 &b) {
-    asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(rec), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
-                 "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w) : "memory");
 }
 
 __global__ void __launch_bounds__(256) fda_sort_clear_kernel(const Problem p) {
@@ -675,6 +670,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 
         __syncwarp();
 
         // the points' own gradients, one point per lane
+        const float scale_x = p.sort_voxel ? p.sort_scale : lv.fW, scale_y = p.sort_voxel ? p.sort_scale : lv.fH;
+        const float scale_z = p.sort_voxel ? p.sort_scale : lv.fD;
         for (int e = lane; e < wn; e += 32) {
             const float4 lo = dots[0][e], hi = dots[1][e], g = geo[e];
             const float x0 = 1.0f - g.x, y0 = 1.0f - g.y, z0 = 1.0f - g.z;
@@ -685,7 +682,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 
             const float s0 = fmaf(g.y, s01, y0 * s00), s1 = fmaf(g.y, s11, y0 * s10);
             const float dx0 = fmaf(g.y, d01, y0 * d00), dx1 = fmaf(g.y, d11, y0 * d10);
             const float gx = fmaf(g.z, dx1, z0 * dx0), gy = fmaf(g.z, s11 - s10, z0 * (s01 - s00)), gz = s1 - s0, da = fmaf(g.z, s1, z0 * s0);
-            __stcs(p.sort_results + w0 + e, make_float4(g.w * lv.fW * gx, g.w * lv.fH * gy, g.w * lv.fD * gz, da));
+            __stcs(p.sort_results + w0 + e, make_float4(g.w * scale_x * gx, g.w * scale_y * gy, g.w * scale_z * gz, da));
         }
         __syncwarp();  // records, units and dot products have been read
         region = next_region;

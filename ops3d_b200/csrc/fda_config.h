@@ -2,6 +2,8 @@
 // on every launch; fda_reload_config() re-reads them (tests change them between calls).
 #pragma once
 
+#include <cuda_runtime.h>
+
 namespace fda {
 
 struct Config {
@@ -22,5 +24,11 @@ const Config &config();
 
 // Remember a failing cudaError_t for fda_last_cuda_error() (per calling thread).
 void record_cuda_error(int cuda_error);
+
+// Parts of the cell-sorted backward that DCNv4 shares (fda_api.cu; kernels in fda_backward_sorted.cuh).
+struct Problem;
+unsigned int sort_scan_tiles(unsigned long long bins);
+int launch_sort_scan(const Problem &p, unsigned long long bins, cudaStream_t st);
+int launch_sort_walk(const Problem &p, int value_dtype, cudaStream_t st);
 
 }  // namespace fda

@@ -79,6 +79,8 @@ struct Problem {
                                    // soft-max probability} {row b*Q*G + q*G + g, unused, element offset of the base corner,
                                    // corner mask}
     float4 *sort_results;          // {d/dx, d/dy, d/dz, dalpha} of every filed point, in list order
+    int sort_voxel;                // results are derivatives by voxel coordinates times sort_scale, not by normalised ones
+    float sort_scale;
 };
 
 constexpr int kMaxSlabs = 128;

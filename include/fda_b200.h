@@ -114,11 +114,15 @@ size_t fda_backward_scratch_bytes(int batch, int num_value, int num_heads, int h
  * The cell-sorted backward (all points sorted by the cell they fall in; gathers and reductions once per run of equal
  * cells instead of once per point) applies to 16-bit values with 16, 32, 48 or 64 channels per head and enough points to pay for
  * its extra launches (FDA_BWD_SORT: 0 off, 1 by size, 2 always).  It needs more scratch than the slab-binned path:
- * fda_backward_sorted_scratch_bytes() (0 when it does not apply).  A caller that wants whichever path the library
- * prefers passes max(fda_backward_scratch_bytes, fda_backward_sorted_scratch_bytes) bytes; fda_backward_workspace_bytes
- * already includes it.  fda_backward_path tells which path such a call takes: 0 the plain scatter kernel, 1 the
- * slab-binned path for the largest level, 2 the cell-sorted path.  No counterpart in the reference.
+ * fda_backward_list_scratch_bytes() (0 when it does not apply); fda_backward_sorted_scratch_bytes() is the same for 32
+ * channels per head and 0 for other widths.  A caller that wants whichever path the library prefers passes
+ * max(fda_backward_scratch_bytes, fda_backward_list_scratch_bytes) bytes; fda_backward_workspace_bytes already includes
+ * it.  fda_backward_path tells which path such a call takes: 0 the plain scatter kernel, 1 the slab-binned path for the
+ * largest level, 2 the cell-sorted path with 32 channels per head, 3 with another width.  The path uses
+ * grad_sampling_loc_attn as scratch until it writes it.  No counterpart in the reference.
  */
+size_t fda_backward_list_scratch_bytes(int batch, int num_value, int num_heads, int head_dim, int num_levels, int num_query,
+                                       int num_points, int value_dtype);
 size_t fda_backward_sorted_scratch_bytes(int batch, int num_value, int num_heads, int head_dim, int num_levels, int num_query,
                                          int num_points, int value_dtype);
 

@@ -16,7 +16,7 @@ DTYPE_CODE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 
 EXPORTS = (
     "fda_status_string", "fda_last_cuda_error", "fda_version", "fda_forward",
-    "fda_backward_workspace_bytes", "fda_backward_scratch_bytes", "fda_backward_sorted_scratch_bytes", "fda_backward_path", "fda_forward_head_group", "fda_backward", "fda_backward_accumulate", "fda_cast_grad_value",
+    "fda_backward_workspace_bytes", "fda_backward_scratch_bytes", "fda_backward_sorted_scratch_bytes", "fda_backward_list_scratch_bytes", "fda_backward_path", "fda_forward_head_group", "fda_backward", "fda_backward_accumulate", "fda_cast_grad_value",
     "fda_backward_noalloc", "fda_peer_reduce_cast", "fda_multimem_reduce_cast", "fda_backward_accumulate_levels",
     "fda_peer_push_partials", "fda_peer_reduce_staged_cast", "fda_backward_bin_plan", "fda_backward_binned_part",
     "fda_pack_sampling", "fda_pack_sampling_backward", "fda_dcnv4_forward", "fda_dcnv4_backward",
@@ -66,8 +66,8 @@ def load() -> ctypes.CDLL:
     lib.fda_backward_path.restype = i
     lib.fda_forward_head_group.argtypes = [i] * 7
     lib.fda_forward_head_group.restype = i
-    lib.fda_backward_sorted_scratch_bytes.argtypes = [i] * 8
-    lib.fda_backward_sorted_scratch_bytes.restype = sz
+    for name in ("fda_backward_sorted_scratch_bytes", "fda_backward_list_scratch_bytes"):
+        getattr(lib, name).argtypes, getattr(lib, name).restype = [i] * 8, sz
     lib.fda_reload_config.restype = None
     lib.fda_backward_touched_rows.argtypes = [i] * 8
     lib.fda_backward_touched_rows.restype = i
@@ -180,7 +180,7 @@ def scratch_bytes(value, packed, K) -> int:
     B, N, G, D = value.shape
     args = (B, N, G, D, _levels(packed, K), packed.shape[1], K)
     return max(int(load().fda_backward_scratch_bytes(*args, DTYPE_CODE[packed.dtype])),
-               int(load().fda_backward_sorted_scratch_bytes(*args, DTYPE_CODE[value.dtype])))
+               int(load().fda_backward_list_scratch_bytes(*args, DTYPE_CODE[value.dtype])))
 
 
 def binning_applies(value, packed, K) -> bool:

@@ -240,8 +240,9 @@ size_t dalpha_plane_bytes(int B, int G, int L, int Q, int K, int pdt) {
     return round256((size_t)B * Q * G * L * K * sizeof(float));
 }
 
-// Cell-sorted backward: [counters] [scan tile sums] [soft-max statistics, 8 bytes per row] [ranks, 4 bytes per point]
-// [entries, 32 bytes per point] [results, 16 bytes per point].  Zero when the path is switched off or the problem does not qualify: 16-bit values with
+// Cell-sorted backward: [where regions start] [spare] [entries, 32 bytes per point] [results, 16 bytes per point].  The
+// counters of the bins and the scan's tile sums live where the results will (the part grows when a sparse problem's
+// counters need more).  Zero when the path is switched off or the problem does not qualify: 16-bit values with
 // 16, 32, 48 or 64 channels per head only (whole k-steps of the walk's matrix products); point ids and list positions are
 // 32-bit; FDA_BWD_SORT=1 wants enough points, below that the extra launches cost more than they save.
 //
@@ -255,9 +256,12 @@ bool sorted_pays(int D, double points, double density) {
     const double sorted = 0.065 + 0.0009 * D + (D <= 32 ? 0.19 : 0.55) / density;
     return points * (plain - sorted) > 70e3;
 }
+// (W+1)(H+1)(D+1) bins per level and head, at most eight times its cells, or a coarse level's spread; and one.
+unsigned long long sort_bins_bound(int B, int N, int G, int L) {
+    return (8ull * N + (unsigned long long)L * fda::kSpreadBins) * B * G + 1;
+}
 struct SortLayout {
-    size_t counters, tile_sums, stats, ranks, entries, results, total;
-    unsigned int tiles;
+    size_t regions, entries, results, counters, tile_sums, total;
 };
 SortLayout sort_layout(int B, int N, int G, int D, int L, int Q, int K, int vdt) {
     SortLayout s;
@@ -265,19 +269,19 @@ SortLayout sort_layout(int B, int N, int G, int D, int L, int Q, int K, int vdt)
     if (g_config.sorted <= 0) return s;
     if (vdt == FDA_DTYPE_F32 || D % 16 != 0 || D > 64) return s;
     if (B <= 0 || N <= 0 || G <= 0 || L <= 0 || Q <= 0 || K <= 0 || (long long)L * G > fda::kWalkRegions) return s;
-    // (W+1)(H+1)(D+1) bins per level and head: at most eight times its cells
-    const unsigned long long bins = 8ull * B * N * G + 1;
-    const unsigned long long points = (unsigned long long)B * Q * G * L * K, rows = (unsigned long long)B * Q * G;
+    const unsigned long long bins = sort_bins_bound(B, N, G, L);
+    const unsigned long long points = (unsigned long long)B * Q * G * L * K;
     if (bins >= (1ull << 31) || points >= (1ull << 31)) return s;
     if (g_config.sorted == 1 && !sorted_pays(D, (double)points, (double)Q * L * K / N)) return s;
-    s.tiles = fda::sort_scan_tiles(bins);
-    s.counters = 0;
-    s.tile_sums = round256(bins * sizeof(unsigned int));
-    s.stats = s.tile_sums + round256((size_t)s.tiles * sizeof(unsigned int));
-    s.ranks = s.stats + round256(rows * sizeof(float2));
-    s.entries = s.ranks + round256(points * sizeof(float));
+    const unsigned long long cells = (unsigned long long)B * N * G, regions = ((unsigned long long)L * G + 1) * B;
+    s.regions = 0;
+    s.entries = round256((cells > regions ? cells : regions) * sizeof(unsigned int)) + round256(fda::sort_scan_tiles(cells) * sizeof(unsigned int));
     s.results = s.entries + round256(points * 2 * sizeof(float4));
-    s.total = s.results + round256(points * sizeof(float4));
+    s.counters = s.results;
+    s.tile_sums = s.counters + round256(bins * sizeof(unsigned int));
+    const size_t scan_end = s.tile_sums + round256(fda::sort_scan_tiles(bins) * sizeof(unsigned int));
+    const size_t results_end = s.results + round256(points * sizeof(float4));
+    s.total = scan_end > results_end ? scan_end : results_end;
     return s;
 }
 
@@ -287,9 +291,9 @@ void attach_sorted(fda::Problem &p, const Shape &s, void *scratch, size_t scratc
     if (lay.total == 0 || scratch_bytes < lay.total) return;
     char *base = static_cast<char *>(scratch);
     p.sort_counters = reinterpret_cast<unsigned int *>(base + lay.counters);
+    p.sort_spread = fda::kSpreadBins;
     p.sort_tile_sums = reinterpret_cast<unsigned int *>(base + lay.tile_sums);
-    p.sort_stats = reinterpret_cast<float2 *>(base + lay.stats);
-    p.sort_ranks = reinterpret_cast<unsigned int *>(base + lay.ranks);
+    p.sort_regions = reinterpret_cast<unsigned int *>(base + lay.regions);
     p.sort_entries = reinterpret_cast<float4 *>(base + lay.entries);
     p.sort_results = reinterpret_cast<float4 *>(base + lay.results);
     p.bin_allowed = 0;  // this layout replaces the binned one
@@ -383,6 +387,12 @@ int launch_binned_part(fda::Problem p, cudaStream_t st) {
     return launch_binned_slabs<VT, PT>(p, st);
 }
 
+// Lanes per row in the count, fill and finalize passes, whatever the channels: four, and eight from 32 points on, where a
+// warp's tile of eight rows leaves too few warps per multiprocessor.  At 40 points per row, 28.7 M points (32 channels) and
+// 45 M (16 channels, two lanes per row before): count 544 -> 360 us and 1390 -> 548, finalize 481 -> 444 and 1783 -> 701; at
+// 24 points, 229.6 M, four lanes are better (count 2.0 against 2.4 ms).
+int sort_lanes_log2(int points_per_row) { return points_per_row >= 32 ? 3 : 2; }
+
 // Exclusive scan of the counters of `bins` bins (an upper bound; the kernels find the real number).
 int launch_scan(const fda::Problem &p, unsigned long long bins, cudaStream_t st) {
     const unsigned int tiles = fda::sort_scan_tiles(bins);
@@ -415,10 +425,11 @@ int launch_sorted(fda::Problem p, cudaStream_t st) {
         return FDA_ERR_BAD_DTYPE;  // not reached: the layout is empty for fp32 values
     } else {
         if (!p.resume) {
-            const unsigned long long bins = 8ull * p.B * p.N * p.G + 1;
+            const unsigned long long bins = sort_bins_bound(p.B, p.N, p.G, p.L);
             const unsigned long long clear_blocks = (bins + 1023) / 1024;
             fda::fda_sort_clear_kernel<<<(unsigned)(clear_blocks > 2368 ? 2368 : clear_blocks), 256, 0, st>>>(p);
             fda::Problem q = p;
+            q.gs_log2 = sort_lanes_log2(p.LK);
             q.row_stride = padded_stride(4 * p.LK);
             const int threads = pick_threads(q, q.row_stride);
             const size_t smem = (size_t)(threads >> q.gs_log2) * q.row_stride * sizeof(float);
@@ -435,6 +446,7 @@ int launch_sorted(fda::Problem p, cudaStream_t st) {
         if (int rc = launch_walk<VT>(p, st)) return rc;
         if (p.finalize) {
             fda::Problem q = p;
+            q.gs_log2 = sort_lanes_log2(p.LK);
             q.row_stride = padded_stride(5 * p.LK);
             const int threads = pick_threads(q, q.row_stride);
             const size_t smem = (size_t)(threads >> q.gs_log2) * q.row_stride * sizeof(float);
@@ -576,6 +588,12 @@ int fda_forward_head_group(int num_value, int num_heads, int head_dim, int num_l
 
 size_t fda_backward_sorted_scratch_bytes(int batch, int num_value, int num_heads, int head_dim, int num_levels, int num_query,
                                          int num_points, int value_dtype) {
+    if (head_dim != 32) return 0;
+    return fda_backward_list_scratch_bytes(batch, num_value, num_heads, head_dim, num_levels, num_query, num_points, value_dtype);
+}
+
+size_t fda_backward_list_scratch_bytes(int batch, int num_value, int num_heads, int head_dim, int num_levels, int num_query,
+                                       int num_points, int value_dtype) {
     return sort_layout(batch, num_value, num_heads, head_dim, num_levels, num_query, num_points, value_dtype).total;
 }
 

@@ -37,14 +37,21 @@ constexpr int kScanTile = kScanItems * kScanThreads;  // counters per scan block
 constexpr unsigned int kNoPosition = 0xffffffffu;     // a point without a corner inside its level
 
 // Bins of one batch element: level l's start at first[l], head g's inside it at g * cells[l].  first[L] = all of them.
+// Bins of a coarse level lie stride[l] counters apart (the ones between stay empty): a level of 21 cells takes 5.7 M atomics
+// on 36 lines otherwise, and those on one line are served one after the other (count pass over 28.7 M points 1055 -> 544 us).
 struct SortBins {
-    unsigned int first[kMaxLevels + 1], cells[kMaxLevels];
+    unsigned int first[kMaxLevels + 1], cells[kMaxLevels], stride[kMaxLevels];
 };
-__device__ __forceinline__ void build_sort_bins(SortBins &s, const int64_t *shapes, int L, int G) {
+constexpr unsigned int kSpreadBins = 4096;  // counters per head that a coarse level is spread over, at most 32 per bin
+__device__ __forceinline__ void build_sort_bins(SortBins &s, const int64_t *shapes, int L, int G, unsigned int spread) {
     unsigned int at = 0;
     for (int l = 0; l < L; ++l) {
+        const unsigned int bins = (unsigned int)(shapes[3 * l] + 1) * (unsigned int)(shapes[3 * l + 1] + 1) * (unsigned int)(shapes[3 * l + 2] + 1);
+        unsigned int stride = 1;
+        while (stride < 32u && bins * stride * 2u <= spread) stride *= 2u;
         s.first[l] = at;
-        s.cells[l] = (unsigned int)(shapes[3 * l] + 1) * (unsigned int)(shapes[3 * l + 1] + 1) * (unsigned int)(shapes[3 * l + 2] + 1);
+        s.stride[l] = stride;
+        s.cells[l] = bins * stride;
         at += s.cells[l] * (unsigned int)G;
     }
     s.first[L] = at;
@@ -72,7 +79,7 @@ __device__ __forceinline__ unsigned int bin_of(const LevelGeom &lv, const BaseCe
 
 __global__ void __launch_bounds__(256) fda_sort_clear_kernel(const Problem p) {
     __shared__ SortBins bins;
-    if (threadIdx.x == 0) build_sort_bins(bins, p.shapes, p.L, p.G);
+    if (threadIdx.x == 0) build_sort_bins(bins, p.shapes, p.L, p.G, p.sort_spread);
     __syncthreads();
     const size_t n = (size_t)bins.first[p.L] * p.B + 1;  // one more: after the scan it holds the length of the list
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; 4 * i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -82,8 +89,13 @@ __global__ void __launch_bounds__(256) fda_sort_clear_kernel(const Problem p) {
     }
 }
 
-// Rank of every point inside its bin, in row order ([row][L*K], kNoPosition for a point that is not filed), and the
-// soft-max statistics {max, 1 / sum} of every row.
+// What the passes tell each other about a row lies where its gradient will: the first 4*L*K of the 8*L*K or more bytes of
+// its row of grad_sampling_loc_attn hold the rank of every point inside its bin, then its position in the list
+// (kNoPosition: not filed); the next eight its soft-max statistics {max, 1 / sum}.
+template <typename PT>
+__device__ __forceinline__ unsigned int *row_slots(const Problem &p, size_t rowg) {
+    return reinterpret_cast<unsigned int *>(static_cast<PT *>(p.grad_packed) + rowg * (size_t)(4 * p.LK));
+}
 template <typename PT>
 __global__ void __launch_bounds__(kThreads) fda_sort_count_kernel(const Problem p) {
     __shared__ LevelGeom geom[kMaxLevels];
@@ -92,7 +104,7 @@ __global__ void __launch_bounds__(kThreads) fda_sort_count_kernel(const Problem 
     const int tid = threadIdx.x;
     if (tid == 0) {
         build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, false, 0ull);
-        build_sort_bins(bins, p.shapes, p.L, p.G);
+        build_sort_bins(bins, p.shapes, p.L, p.G, p.sort_spread);
     }
     const int b = blockIdx.y;
     const int gs = 1 << p.gs_log2;
@@ -119,7 +131,8 @@ __global__ void __launch_bounds__(kThreads) fda_sort_count_kernel(const Problem 
     float s = 0.f;
     for (int i = lane_c; i < LK; i += gs) s += row_ok ? __expf(trow[3 * LK + i] - m) : 0.f;
     for (int mask = gs >> 1; mask > 0; mask >>= 1) s += __shfl_xor_sync(0xffffffffu, s, mask);
-    if (row_ok && lane_c == 0) p.sort_stats[(size_t)b * p.rows_per_b + row] = make_float2(m, 1.0f / s);
+    if (row_ok && lane_c == 0)
+        *reinterpret_cast<float2 *>(row_slots<PT>(p, (size_t)b * p.rows_per_b + row) + LK) = make_float2(m, 1.0f / s);
     // Eight points at a time: all requests go out before the first answer is needed.  The ranks take the place of the
     // logits in the tile (a lane overwrites only slots it owns).
     constexpr int kBatch = 8;
@@ -133,7 +146,7 @@ __global__ void __launch_bounds__(kThreads) fda_sort_count_kernel(const Problem 
                 const int l = (i >> 2) >> p.k_shift;
                 const LevelGeom lv = geom[l];
                 const BaseCell c = base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2]);
-                if (c.ok) rank[u] = atomicAdd(counters + bins.first[l] + g * bins.cells[l] + bin_of(lv, c), 1u);
+                if (c.ok) rank[u] = atomicAdd(counters + bins.first[l] + g * bins.cells[l] + bin_of(lv, c) * bins.stride[l], 1u);
             }
         }
 #pragma unroll
@@ -143,12 +156,12 @@ __global__ void __launch_bounds__(kThreads) fda_sort_count_kernel(const Problem 
         }
     }
     __syncwarp();
-    float *dst = reinterpret_cast<float *>(p.sort_ranks) + ((size_t)b * p.rows_per_b + first) * (size_t)LK;
     const float inv_vec = 4.0f / (float)LK;
     for (int v = lane; v < nrows * (LK >> 2); v += 32) {
         const int r = row_of_vector(v, inv_vec);
         const int c = (v - r * (LK >> 2)) * 4;
-        *reinterpret_cast<float4 *>(dst + (size_t)v * 4) = *reinterpret_cast<const float4 *>(wtile + r * p.row_stride + 3 * LK + c);
+        *reinterpret_cast<float4 *>(row_slots<PT>(p, (size_t)b * p.rows_per_b + first + r) + c) =
+            *reinterpret_cast<const float4 *>(wtile + r * p.row_stride + 3 * LK + c);
     }
 }
 
@@ -162,7 +175,7 @@ __global__ void __launch_bounds__(kThreads) fda_sort_fill_kernel(const Problem p
     const int tid = threadIdx.x;
     if (tid == 0) {
         build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, false, 0ull);
-        build_sort_bins(bins, p.shapes, p.L, p.G);
+        build_sort_bins(bins, p.shapes, p.L, p.G, p.sort_spread);
     }
     const int b = blockIdx.y;
     const int gs = 1 << p.gs_log2;
@@ -179,13 +192,17 @@ __global__ void __launch_bounds__(kThreads) fda_sort_fill_kernel(const Problem p
     stage_rows<PT>(static_cast<const PT *>(p.packed) + ((size_t)b * p.rows_per_b + first) * (size_t)(4 * LK), wtile, nrows,
                    LK, p.row_stride, lane);
     __syncthreads();  // level table and this warp's tile visible
+    const unsigned int *starts = p.sort_counters + (size_t)b * bins.first[p.L];
+    if (blockIdx.x == 0)  // the walk overwrites the counters with its results; it needs where regions start
+        for (int r = tid; r <= p.L * p.G; r += blockDim.x)
+            p.sort_regions[(size_t)b * (p.L * p.G + 1) + r] =
+                starts[r < p.L * p.G ? bins.first[r / p.G] + (unsigned int)(r % p.G) * bins.cells[r / p.G] : bins.first[p.L]];
     if (row >= p.rows_per_b) return;
     const float *trow = wtile + (lane >> p.gs_log2) * p.row_stride;
     const unsigned int g = (unsigned int)(row % p.G);
     const size_t rowg = (size_t)b * p.rows_per_b + row;
-    const unsigned int *starts = p.sort_counters + (size_t)b * bins.first[p.L];
-    unsigned int *ranks = p.sort_ranks + rowg * (size_t)LK;
-    const float2 stats = __ldg(p.sort_stats + rowg);
+    unsigned int *ranks = row_slots<PT>(p, rowg);
+    const float2 stats = *reinterpret_cast<const float2 *>(ranks + LK);
     constexpr int kBatch = 4;  // the starts of four points are requested before the first is used
     for (int i0 = lane_c; i0 < LK; i0 += kBatch * gs) {
         unsigned int pos[kBatch], start[kBatch];
@@ -197,7 +214,8 @@ __global__ void __launch_bounds__(kThreads) fda_sort_fill_kernel(const Problem p
             if (pos[u] != kNoPosition) {
                 const int l = (i >> 2) >> p.k_shift;
                 const LevelGeom lv = geom[l];
-                start[u] = __ldg(starts + bins.first[l] + g * bins.cells[l] + bin_of(lv, base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2])));
+                start[u] = __ldg(starts + bins.first[l] + g * bins.cells[l] +
+                                 bin_of(lv, base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2])) * bins.stride[l]);
             }
         }
 #pragma unroll
@@ -252,7 +270,7 @@ __device__ __forceinline__ unsigned int block_exclusive_scan(unsigned int v, uns
 // The host sizes the counters for the most bins a volume of N cells can have; the kernels find the real number.
 __device__ __forceinline__ size_t counters_of(const Problem &p) {
     SortBins bins;
-    build_sort_bins(bins, p.shapes, p.L, p.G);
+    build_sort_bins(bins, p.shapes, p.L, p.G, p.sort_spread);
     return (size_t)bins.first[p.L] * p.B + 1;
 }
 
@@ -432,19 +450,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 
     const int level_begin = __ffs(p.level_mask) - 1, level_end = 32 - __clz(p.level_mask);  // a contiguous range
     const int regions = (level_end - level_begin) * p.G;
     if (tid == 0) build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, true, p.l2_keep_bytes);
-    {
-        SortBins bins;
-        build_sort_bins(bins, p.shapes, p.L, p.G);
-        const unsigned int *starts = p.sort_counters + (size_t)b * bins.first[p.L];
-        for (int r = tid; r <= regions; r += blockDim.x) {
-            unsigned int bin = bins.first[level_end];
-            if (r < regions) {
-                const int l = level_begin + r / p.G;
-                bin = bins.first[l] + (unsigned int)(r % p.G) * bins.cells[l];
-            }
-            region_entry[r] = starts[bin];
-        }
-    }
+    for (int r = tid; r <= regions; r += blockDim.x) region_entry[r] = p.sort_regions[(size_t)b * (p.L * p.G + 1) + level_begin * p.G + r];
     __syncthreads();
     if (warp == 0) {
         unsigned int carry = 0;
@@ -712,9 +718,9 @@ __global__ void __launch_bounds__(kThreads) fda_sort_finalize_kernel(const Probl
     nrows = nrows < 0 ? 0 : (nrows > rows_per_warp ? rows_per_warp : nrows);
     float *trow = wtile + (lane >> p.gs_log2) * p.row_stride;
     const size_t rowg = (size_t)b * p.rows_per_b + (row_ok ? row : 0);
-    const unsigned int *positions = p.sort_ranks + rowg * (size_t)LK;
+    const unsigned int *positions = row_slots<PT>(p, rowg);  // all read before the first gradient of the row is written
     const PT *logits = static_cast<const PT *>(p.packed) + rowg * (size_t)(4 * LK) + 3 * LK;
-    const float2 stats = __ldg(p.sort_stats + rowg);
+    const float2 stats = *reinterpret_cast<const float2 *>(positions + LK);
 
     // Tile row: [0,3LK) coordinate gradients, [3LK,4LK) dalpha -> logit gradients, [4LK,5LK) probabilities.
     float S = 0.f;

@@ -254,7 +254,7 @@ constexpr unsigned int kSortNone = 0xffffffffu;       // no corner inside the vo
 constexpr unsigned int kSortNotFinite = 0xfffffff0u;  // the same, and axes (bits x, y, z) whose position is not finite
 
 struct DcnSort {
-    unsigned int *counters, *ranks;
+    unsigned int *counters, *ranks, *regions;
     float2 *stats;
     float4 *entries, *results;
     int64_t *shape;  // d, h, w of the volume, 0 (the one level's extents and start)
@@ -377,6 +377,8 @@ __global__ void __launch_bounds__(fda::kThreads) dcnv4_sort_fill_kernel(const Dc
     const unsigned int cells = (unsigned int)(p.Din + 1) * (unsigned int)(p.Hin + 1) * (unsigned int)(p.Win + 1);
     const unsigned int *starts = s.counters + (size_t)b * p.G * cells;
     unsigned int *ranks = s.ranks + ((size_t)b * p.rows_per_b + rows.first) * (size_t)K;
+    if (blockIdx.x == 0)
+        for (int g = threadIdx.x; g <= p.G; g += blockDim.x) s.regions[(size_t)b * (p.G + 1) + g] = starts[(size_t)g * cells];
     const uint32_t sx = (uint32_t)p.GD, sy = (uint32_t)p.Win * sx, sz = (uint32_t)p.Hin * sy;
     const float inv_k = 1.0f / (float)K;
     const int n = rows.nrows * K;
@@ -538,11 +540,11 @@ bool dcn_sorted_pays(int D, double points, double density) {
     return points * (plain - sorted) > 40e3;
 }
 
-// Scratch of the cell-sorted backward, behind the fp32 image: [shape] [counters] [scan tile sums] [soft-max statistics]
-// [ranks] [entries] [results], 52 bytes per point; total 0 when the path is not taken.  A call is sorted `elements` batch
+// Scratch of the cell-sorted backward, behind the fp32 image: [shape] [where groups start] [counters] [scan tile sums]
+// [soft-max statistics] [ranks] [entries] [results], 52 bytes per point; total 0 when the path is not taken.  A call is sorted `elements` batch
 // elements at a time, as many as keep the list at 32 M points (at least one), which bounds the scratch.
 struct DcnSortLayout {
-    size_t shape, counters, tile_sums, stats, ranks, entries, results, total;
+    size_t shape, regions, counters, tile_sums, stats, ranks, entries, results, total;
     int elements;
 };
 DcnSortLayout dcn_sort_layout(const DcnProblem &p, int dtype) {
@@ -563,7 +565,8 @@ DcnSortLayout dcn_sort_layout(const DcnProblem &p, int dtype) {
     const unsigned long long counters = elements * bins + 1;
     const size_t n = (size_t)(elements * points), rows = (size_t)elements * p.rows_per_b;
     s.shape = 0;
-    s.counters = 256;
+    s.regions = 256;
+    s.counters = s.regions + round256((size_t)elements * (p.G + 1) * sizeof(unsigned int));
     s.tile_sums = s.counters + round256(counters * sizeof(unsigned int));
     s.stats = s.tile_sums + round256(fda::sort_scan_tiles(counters) * sizeof(unsigned int));
     s.ranks = s.stats + round256(rows * sizeof(float2));
@@ -578,6 +581,7 @@ int launch_dcn_sorted(const DcnProblem &p0, const DcnSortLayout &lay, char *scra
     DcnSort s;
     s.shape = reinterpret_cast<int64_t *>(scratch + lay.shape);
     s.counters = reinterpret_cast<unsigned int *>(scratch + lay.counters);
+    s.regions = reinterpret_cast<unsigned int *>(scratch + lay.regions);
     s.stats = reinterpret_cast<float2 *>(scratch + lay.stats);
     s.ranks = reinterpret_cast<unsigned int *>(scratch + lay.ranks);
     s.entries = reinterpret_cast<float4 *>(scratch + lay.entries);
@@ -608,7 +612,7 @@ int launch_dcn_sorted(const DcnProblem &p0, const DcnSortLayout &lay, char *scra
         w.B = p.B; w.N = (int)cells; w.G = p.G; w.D = p.D; w.L = 1; w.K = p.K; w.Q = p.Q; w.LK = p.K;
         w.rows_per_b = p.rows_per_b; w.GD = p.GD; w.gs_log2 = p.gs_log2; w.lpg = p.lpg; w.head_group = p.G;
         w.l2_keep_bytes = p.l2_keep_bytes; w.value_elem_bytes = sizeof(T); w.level_mask = 1;
-        w.sort_counters = s.counters; w.sort_stats = s.stats; w.sort_ranks = s.ranks; w.sort_entries = s.entries;
+        w.sort_counters = s.counters; w.sort_regions = s.regions; w.sort_entries = s.entries;
         w.sort_tile_sums = reinterpret_cast<unsigned int *>(scratch + lay.tile_sums);
         w.sort_results = s.results;
         w.sort_voxel = 1; w.sort_scale = p.offset_scale;

@@ -72,9 +72,9 @@ struct Problem {
     float *dalpha;
     // backward, cell-sorted handling of all levels (see fda_backward_sorted.cuh); null: not used
     unsigned int *sort_counters;   // per (batch, level, head, base cell): points -> exclusive scan; then the length of the list
+    unsigned int sort_spread;      // counters per head that a coarse level's bins are spread over (0: one next to the other)
     unsigned int *sort_tile_sums;  // scratch of the scan
-    float2 *sort_stats;            // [B*Q*G]: soft-max statistics {max, 1 / sum} of every row
-    unsigned int *sort_ranks;      // [B*Q*G][L*K]: rank of a point inside its bin -> its position in the list
+    unsigned int *sort_regions;    // [B][L*G+1]: where the list of every level and head starts, and the end
     float4 *sort_entries;          // sorted list, 32 bytes per point: {fractions of the voxel position along x, y, z,
                                    // soft-max probability} {row b*Q*G + q*G + g, unused, element offset of the base corner,
                                    // corner mask}

@@ -247,15 +247,19 @@ size_t dalpha_plane_bytes(int B, int G, int L, int Q, int K, int pdt) {
 // 32-bit; FDA_BWD_SORT=1 wants enough points, below that the extra launches cost more than they save.
 //
 // Whether it pays: measured per point, the plain scatter takes 0.12 / 0.155 / 0.375 ns with 2 / 4 / 8 lanes per row, the
-// sorted one 0.065 + 0.0009 D plus what a run costs (0.19 ns, 0.55 above 32 channels) over the points per run, about the
-// density of points per cell and head; its eight launches cost 70 us more than the three of the plain path.  At 32
-// channels that is 2.4 M points at a density of 4, 1.2 M at 16 (73728 cells: 398 -> 388 us at 2.4 M, 742 -> 583 at 4.7 M,
-// 1426 -> 990 at 9.4 M; 64 channels 955 -> 664, 1805 -> 945, 3526 -> 1477).
+// sorted one 0.065 + 0.0009 D plus what a run costs (0.29 ns, 0.55 above 32 channels) over the points per run, about the
+// density of points per cell and head; its eight launches cost 70 us more than the three of the plain path (90 above 32
+// channels).  These are the costs of points spread over the whole volume; where every query samples around its own cell both
+// are cheaper, and at 16 channels the plain scatter gains more by it (density 16: spread 6.6 M points 810 -> 603 us, local
+// 6.2 M 388 -> 410, 11.5 M 945 -> 985; 20.8 M at 32 1656 -> 1503), hence the higher line there.  32 channels: density 4, 5.7 M
+// points 966 -> 1173 us; 8, 2.7 M 400 -> 425, 4.7 M 742 -> 583; 16, 1.6 M 298 -> 216, 24.8 M 3574 -> 2526.  64 channels,
+// density 8: 0.4 M 104 -> 120 us, 0.9 M 257 -> 235.
 bool sorted_pays(int D, double points, double density) {
     const double plain = D <= 16 ? 0.12 : (D <= 32 ? 0.155 : 0.375);
-    const double sorted = 0.065 + 0.0009 * D + (D <= 32 ? 0.19 : 0.55) / density;
-    return points * (plain - sorted) > 70e3;
+    const double sorted = 0.065 + 0.0009 * D + (D <= 32 ? 0.29 : 0.55) / density;
+    return points * (plain - sorted) > (D <= 16 ? 300e3 : (D <= 32 ? 70e3 : 90e3));
 }
+
 // (W+1)(H+1)(D+1) bins per level and head, at most eight times its cells, or a coarse level's spread; and one.
 unsigned long long sort_bins_bound(int B, int N, int G, int L) {
     return (8ull * N + (unsigned long long)L * fda::kSpreadBins) * B * G + 1;

@@ -38,6 +38,7 @@ struct DcnProblem {
     float offset_scale;
     int remove_center, softmax;
     int gs_log2, lpg, rows_per_b, GD, row_stride;
+    int vector_rows;         // offset rows (and their gradients) start on a boundary of four values
     unsigned long long l2_keep_bytes;
 };
 
@@ -79,7 +80,15 @@ __device__ __forceinline__ void stage_dcn_rows(const DcnProblem &p, int b, int f
     for (int r = 0; r < nrows; ++r) {
         const int row = first_row + r, q = row / p.G, g = row - q * p.G;
         const T *src = base + (size_t)q * p.padded + (size_t)g * per_row;
-        for (int e = lane; e < per_row; e += 32) wtile[r * p.row_stride + e] = fda::load1<T>(src + e);
+        float *dst = wtile + r * p.row_stride;
+        if (p.vector_rows) {  // four values per load, one load per lane for 27 points: forward of 56.6 M points 2.85 -> 2.62 ms
+            for (int e = 4 * lane; e < per_row; e += 128) {
+                const float4 v = fda::load4<T>(src + e);
+                dst[e] = v.x; dst[e + 1] = v.y; dst[e + 2] = v.z; dst[e + 3] = v.w;
+            }
+        } else {
+            for (int e = lane; e < per_row; e += 32) dst[e] = fda::load1<T>(src + e);
+        }
     }
 }
 
@@ -269,6 +278,17 @@ struct SortRows {
     int first, nrows;
     float *tile;
 };
+// Stencil positions times dilation, by point, in front of the tiles: two integer divisions per point otherwise.  Whole block.
+__device__ __forceinline__ float *stencil_table(const DcnProblem &p, float *smem) {
+    for (int k = threadIdx.x; k < p.K; k += blockDim.x) {
+        const int kk = k + (p.remove_center && k >= ((p.kw / 2) * p.kh + p.kh / 2) * p.kd + p.kd / 2 ? 1 : 0);
+        const int ij = kk / p.kd, i = ij / p.kh;
+        smem[3 * k] = (float)(i * p.dw);
+        smem[3 * k + 1] = (float)((ij - i * p.kh) * p.dh);
+        smem[3 * k + 2] = (float)((kk - ij * p.kd) * p.dd);
+    }
+    return smem;
+}
 // Stages the warp's rows and each row's stencil base and group.
 template <typename T>
 __device__ __forceinline__ SortRows sort_rows(const DcnProblem &p, float *smem, int b) {
@@ -295,13 +315,11 @@ struct DcnCell {
     unsigned int code;  // 0: at least one corner inside
     unsigned int bin;   // inside the group
 };
-__device__ __forceinline__ DcnCell dcn_cell(const DcnProblem &p, const float *trow, int k) {
-    const int kk = k + (p.remove_center && k >= ((p.kw / 2) * p.kh + p.kh / 2) * p.kd + p.kd / 2 ? 1 : 0);
-    const int ij = kk / p.kd, i = ij / p.kh;
+__device__ __forceinline__ DcnCell dcn_cell(const DcnProblem &p, const float *stencil, const float *trow, int k) {
     const float *extra = trow + 4 * p.K;
-    const float x = __fmaf_rn(__fadd_rn((float)(i * p.dw), trow[3 * k]), p.offset_scale, extra[0]);
-    const float y = __fmaf_rn(__fadd_rn((float)((ij - i * p.kh) * p.dh), trow[3 * k + 1]), p.offset_scale, extra[1]);
-    const float z = __fmaf_rn(__fadd_rn((float)((kk - ij * p.kd) * p.dd), trow[3 * k + 2]), p.offset_scale, extra[2]);
+    const float x = __fmaf_rn(__fadd_rn(stencil[3 * k], trow[3 * k]), p.offset_scale, extra[0]);
+    const float y = __fmaf_rn(__fadd_rn(stencil[3 * k + 1], trow[3 * k + 1]), p.offset_scale, extra[1]);
+    const float z = __fmaf_rn(__fadd_rn(stencil[3 * k + 2], trow[3 * k + 2]), p.offset_scale, extra[2]);
     const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
     DcnCell c;
     c.x = (int)xf; c.y = (int)yf; c.z = (int)zf;  // saturates; NaN is cell 0, its weights stay NaN
@@ -320,8 +338,9 @@ template <typename T>
 __global__ void __launch_bounds__(fda::kThreads) dcnv4_sort_count_kernel(const DcnProblem p, const DcnSort s) {
     extern __shared__ __align__(16) float smem_tile[];
     const int lane = threadIdx.x & 31, b = blockIdx.y, K = p.K;
-    const SortRows rows = sort_rows<T>(p, smem_tile, b);
-    __syncwarp();
+    const float *stencil = stencil_table(p, smem_tile);
+    const SortRows rows = sort_rows<T>(p, smem_tile + 3 * p.K, b);
+    __syncthreads();
     {   // soft-max statistics, four lanes per row
         const int r = lane >> 2;
         const float *trow = rows.tile + r * p.row_stride + 3 * K;
@@ -352,7 +371,7 @@ __global__ void __launch_bounds__(fda::kThreads) dcnv4_sort_count_kernel(const D
             if (e < n) {
                 const int r = fda::row_of_vector(e, inv_k);
                 const float *trow = rows.tile + r * p.row_stride;
-                const DcnCell c = dcn_cell(p, trow, e - r * K);
+                const DcnCell c = dcn_cell(p, stencil, trow, e - r * K);
                 rank[u] = c.code;
                 if (c.code == 0u) rank[u] = atomicAdd(counters + (size_t)__float_as_int(trow[4 * K + 5]) * cells + c.bin, 1u);
             }
@@ -367,13 +386,14 @@ template <typename T>
 __global__ void __launch_bounds__(fda::kThreads) dcnv4_sort_fill_kernel(const DcnProblem p, const DcnSort s) {
     extern __shared__ __align__(16) float smem_tile[];
     const int lane = threadIdx.x & 31, b = blockIdx.y, K = p.K;
-    const SortRows rows = sort_rows<T>(p, smem_tile, b);
+    const float *stencil = stencil_table(p, smem_tile);
+    const SortRows rows = sort_rows<T>(p, smem_tile + 3 * p.K, b);
     if (lane < rows.nrows) {
         const float2 st = s.stats[(size_t)b * p.rows_per_b + rows.first + lane];
         float *extra = rows.tile + lane * p.row_stride + 4 * K;
         extra[3] = st.x; extra[4] = st.y;
     }
-    __syncwarp();
+    __syncthreads();
     const unsigned int cells = (unsigned int)(p.Din + 1) * (unsigned int)(p.Hin + 1) * (unsigned int)(p.Win + 1);
     const unsigned int *starts = s.counters + (size_t)b * p.G * cells;
     unsigned int *ranks = s.ranks + ((size_t)b * p.rows_per_b + rows.first) * (size_t)K;
@@ -387,7 +407,7 @@ __global__ void __launch_bounds__(fda::kThreads) dcnv4_sort_fill_kernel(const Dc
         if (rank >= kSortNotFinite) continue;
         const int r = fda::row_of_vector(e, inv_k), k = e - r * K;
         const float *trow = rows.tile + r * p.row_stride;
-        const DcnCell c = dcn_cell(p, trow, k);
+        const DcnCell c = dcn_cell(p, stencil, trow, k);
         const unsigned int at = starts[(size_t)__float_as_int(trow[4 * K + 5]) * cells + c.bin] + rank;
         const unsigned int mx = (unsigned int)(c.x >= 0) | (unsigned int)(c.x + 1 < p.Win) << 1;    // corners dx = 0, 1
         const unsigned int mxy = (c.y >= 0 ? mx : 0u) | (c.y + 1 < p.Hin ? mx << 2 : 0u);          // dy*2 + dx
@@ -462,7 +482,11 @@ __global__ void __launch_bounds__(fda::kThreads) dcnv4_sort_finalize_kernel(cons
     for (int r = 0; r < nrows; ++r) {
         const int row = first + r, q = row / p.G, g = row - q * p.G;
         T *dst = gbase + (size_t)q * p.padded + (size_t)g * per_row;
-        for (int e = lane; e < per_row; e += 32) fda::store1<T>(dst + e, tile[r * p.row_stride + e]);
+        const float *src = tile + r * p.row_stride;
+        if (p.vector_rows)
+            for (int e = 4 * lane; e < per_row; e += 128) fda::store4_stream<T>(dst + e, make_float4(src[e], src[e + 1], src[e + 2], src[e + 3]));
+        else
+            for (int e = lane; e < per_row; e += 32) fda::store1<T>(dst + e, src[e]);
     }
 }
 
@@ -597,8 +621,8 @@ int launch_dcn_sorted(const DcnProblem &p0, const DcnSortLayout &lay, char *scra
         p.grad_offset = static_cast<T *>(p0.grad_offset) + (size_t)b0 * p0.Q * p0.padded;
         p.row_stride = (4 * p.K + kRowExtra) | 1;  // odd: the rows of a warp start in different banks
         int warps = fda::kThreads / 32;
-        while (warps > 1 && (size_t)warps * kSortRows * p.row_stride * sizeof(float) > 48 * 1024) warps >>= 1;
-        const size_t smem = (size_t)warps * kSortRows * p.row_stride * sizeof(float);  // K <= 125: at most 16.3 KB per warp
+        while (warps > 1 && ((size_t)warps * kSortRows * p.row_stride + 3 * p.K) * sizeof(float) > 48 * 1024) warps >>= 1;
+        const size_t smem = ((size_t)warps * kSortRows * p.row_stride + 3 * p.K) * sizeof(float);  // K <= 125: at most 16.3 KB per warp
         const int rows_per_block = warps * kSortRows;
         const dim3 grid((unsigned)((p.rows_per_b + rows_per_block - 1) / rows_per_block), (unsigned)p.B, 1);
         const size_t bins = (size_t)(p.Din + 1) * (p.Hin + 1) * (p.Win + 1) * p.G * p.B + 1;
@@ -632,6 +656,11 @@ int dispatch_dcn(const DcnProblem &p, int dtype, bool backward, cudaStream_t st)
     return launch_dcn<__nv_bfloat16>(p, backward, st);
 }
 
+// A row's blocks of 4 * K values start at multiples of four values.
+inline bool rows_aligned(const void *rows, int padded, int dtype) {
+    return padded % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & (uintptr_t)(4 * dtype_size(dtype) - 1)) == 0;
+}
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -658,6 +687,7 @@ extern "C" int fda_dcnv4_forward(const void *value, const void *p_offset, void *
         return rc;
     if (!aligned16(value) || !aligned16(output)) return FDA_ERR_MISALIGNED;
     p.value = value; p.offset = p_offset; p.out = output;
+    p.vector_rows = rows_aligned(p_offset, padded_offset_dim, dtype);
     return dispatch_dcn(p, dtype, false, static_cast<cudaStream_t>(stream));
 }
 
@@ -707,6 +737,7 @@ extern "C" int fda_dcnv4_backward(const void *value, const void *p_offset, const
                               0, (size_t)(padded_offset_dim - used) * dtype_size(dtype), (size_t)batch * p.Q, st);
     if (e != cudaSuccess) { fda::record_cuda_error((int)e); return FDA_ERR_CUDA; }
     p.value = value; p.offset = p_offset; p.grad_out = grad_output; p.accum = accum; p.grad_offset = grad_offset;
+    p.vector_rows = rows_aligned(p_offset, padded_offset_dim, dtype) && rows_aligned(grad_offset, padded_offset_dim, dtype);
     const DcnSortLayout lay = dcn_sort_layout(p, dtype);
     if (lay.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && workspace_bytes >= round256(need) + lay.total) {
         char *scratch = static_cast<char *>(workspace) + round256(need);

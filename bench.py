@@ -663,7 +663,7 @@ def run_ours(args, cfg):
         "bound": "hbm",
         "kernel": "backward pass (one C-ABI call) = " + ("fda_touch_rows_kernel (zeroes the image rows the points touch) + "
                                                          if touched else "zero-fill + ") + {
-            2: "cell sort (fda_sort_pass_kernel count / fill, fda_scan_*) + fda_sorted_walk_kernel + fda_sort_finalize_kernel",
+            2: "cell sort (fda_sort_clear / count / fill kernels, fda_scan_*) + fda_sorted_walk_kernel + fda_sort_finalize_kernel",
             1: "slab binning + fda_backward_binned_kernel + fda_backward_kernel",
             0: "fda_backward_kernel"}[bwd_path],
         "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

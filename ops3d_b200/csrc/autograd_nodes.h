@@ -4,9 +4,9 @@
 // 91 us (the function's bookkeeping, two launch-hint searches that the kernels ignore, and the GIL for the engine's
 // thread in the backward).  As nodes, a call is one binding call in each direction and the backward never enters Python.
 //
-// Semantics are those of a Python Function with once_differentiable: inputs are saved with version checks and saved-tensor
-// hooks, a second backward without retain_graph raises, and differentiating the gradients raises (where the Python
-// version raised).
+// Semantics are those of a Python Function with once_differentiable in reverse mode on plain tensors: inputs are saved with
+// version checks and saved-tensor hooks, a second backward without retain_graph raises, and differentiating the gradients
+// raises (where the Python version raised).  Every other mode takes the Python Function (ops3d_b200/graph.py).
 #pragma once
 
 #include <torch/csrc/autograd/function.h>

@@ -12,8 +12,10 @@ reference ``csrc/dcnv4.h:7-61``); the same two functions, with the same position
 from __future__ import annotations
 
 from torch.autograd import Function
+from torch.autograd.function import once_differentiable
 
 from ._extension import _C, _C_IMPORT_ERROR
+from .graph import takes_node
 
 
 def _ext():
@@ -24,10 +26,28 @@ def _ext():
 
 class DCNv4Function(Function):
     """``apply(value, p_offset, kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step,
-    remove_center, softmax)``; ``kernel`` .. ``dilation`` are (d, h, w) triples."""
+    remove_center, softmax)``; ``kernel`` .. ``dilation`` are (d, h, w) triples.  ``apply`` is a C++ graph node, ``forward`` and
+    ``backward`` what it does where something has to see the Function itself (``graph.takes_node``)."""
 
     @staticmethod
-    def apply(value, p_offset, kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step=64, remove_center=0,
+    def forward(ctx, value, p_offset, kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step=64,
+                remove_center=0, softmax=False):
+        ctx.shape = (*kernel, *stride, *pad, *dilation, group, group_channels, float(offset_scale), im2col_step)
+        ctx.masks = (int(remove_center), 8, 0, bool(softmax))
+        ctx.save_for_backward(value, p_offset)
+        return _ext().dcnv4_forward(value, p_offset, *ctx.shape, *ctx.masks)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, grad_output):
+        grads = _ext().dcnv4_backward(*ctx.saved_tensors, *ctx.shape, grad_output.contiguous(), *ctx.masks)
+        return (*grads, *(None,) * 10)
+
+    @classmethod
+    def apply(cls, value, p_offset, kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step=64, remove_center=0,
               softmax=False):
-        return _ext().dcnv4(value, p_offset, kernel, stride, pad, dilation, group, group_channels, float(offset_scale), im2col_step,
-                            int(remove_center), bool(softmax))
+        if cls is DCNv4Function and takes_node():
+            return _ext().dcnv4(value, p_offset, kernel, stride, pad, dilation, group, group_channels, float(offset_scale), im2col_step,
+                                int(remove_center), bool(softmax))
+        return super().apply(value, p_offset, kernel, stride, pad, dilation, group, group_channels, offset_scale, im2col_step,
+                             remove_center, softmax)

@@ -20,8 +20,10 @@ the kernels treat the results as hints and ignore them, so the operator itself d
 from __future__ import annotations
 
 from torch.autograd import Function
+from torch.autograd.function import once_differentiable
 
 from ._extension import _C, _C_IMPORT_ERROR
+from .graph import takes_node
 
 
 def _require_extension():
@@ -69,10 +71,33 @@ def findspec_bwd(B, Q, G, C, max_tpb=256, max_mult=64):
 
 
 class FlashDeformAttnFunction(Function):
-    """The differentiable operator.  Forward, saved tensors and backward are a C++ graph node (``csrc/autograd_nodes.h``):
-    gradients reach ``value`` and ``sampling_loc_attn``, once (differentiating them raises)."""
+    """The differentiable operator: gradients reach ``value`` and ``sampling_loc_attn``, once (differentiating them raises).
+
+    ``apply`` is a C++ graph node with these semantics (``csrc/autograd_nodes.h``); ``forward`` and ``backward`` are what it
+    does where something has to see the Function itself (``graph.takes_node``) and in subclasses."""
 
     @staticmethod
-    def apply(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn, im2col_step, K=8, use_reg=True):
-        return _require_extension().flash_deform_attn(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn,
-                                                      im2col_step, K, use_reg)
+    def forward(ctx, value, value_spatial_shapes, value_level_start_index, sampling_loc_attn, im2col_step, K=8, use_reg=True):
+        ext = _require_extension()
+        L, last = value_spatial_shapes.shape[0], sampling_loc_attn.shape[-1]
+        if last != L * K * 4:
+            raise ValueError(f"sampling_loc_attn last dimension ({last}) does not match value_spatial_shapes level count "
+                             f"L={L} and K={K} (expected {L * K * 4})")
+        B, Q, G, C = value.shape[0], sampling_loc_attn.shape[1], value.shape[2], value.shape[3]
+        ctx.args = (im2col_step, K, *findspec_bwd(B, Q, G, C))
+        ctx.save_for_backward(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn)
+        return ext.flash_deform_attn_forward(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn,
+                                             im2col_step, K, *findspec(B, Q, G, C), use_reg)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, grad_output):
+        grad_value, grad_packed = _require_extension().flash_deform_attn_backward(*ctx.saved_tensors, grad_output.contiguous(), *ctx.args)
+        return grad_value, None, None, grad_packed, None, None, None
+
+    @classmethod
+    def apply(cls, value, value_spatial_shapes, value_level_start_index, sampling_loc_attn, im2col_step, K=8, use_reg=True):
+        if cls is FlashDeformAttnFunction and takes_node():
+            return _require_extension().flash_deform_attn(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn,
+                                                          im2col_step, K, use_reg)
+        return super().apply(value, value_spatial_shapes, value_level_start_index, sampling_loc_attn, im2col_step, K, use_reg)

@@ -100,3 +100,15 @@ def test_forward_mode_raises(make, binding):
             call(function.apply, dual)
         assert torch.equal(call(function.apply, x), call(function.apply, x))  # plain tensors go on as usual
     assert binding.nodes == 0
+
+
+@pytest.mark.parametrize("make", OPS)
+@pytest.mark.parametrize("grad", [False, True])
+def test_a_traced_call_runs_on_new_inputs(make, grad, binding):
+    function, x, call = make()
+    with torch.set_grad_enabled(grad):
+        traced = torch.jit.trace(lambda v: call(function.apply, v), (x,), check_trace=False)
+        assert binding.nodes == 0
+        other = x + 1
+        assert torch.allclose(traced(other), call(function.apply, other))
+        assert not torch.allclose(traced(other), traced(x))

@@ -90,7 +90,9 @@ def build_binding(force: bool = False, verbose: bool = False) -> str:
         os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
         "-DTORCH_EXTENSION_NAME=_C", "-DTORCH_API_INCLUDE_EXTENSION_H",
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-        *inc, src, "-o", EXT,
+        # the process's libstdc++ by name: a compiler that finds only the archive would link a second copy of it, and the
+        # first message with a number in it then crashes in that copy's locales
+        *inc, src, "-o", EXT, "-l:libstdc++.so.6",
         f"-L{PKG}", "-lfda_b200", "-Wl,-rpath,$ORIGIN",
     ]
     for d in libdirs:

@@ -64,3 +64,10 @@ def test_saved_inputs_are_version_checked(make):
         copies[0].mul_(2)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out.sum().backward()
+
+
+def test_an_error_message_with_numbers_raises():
+    value, offset = torch.randn(1, 2, 2, 2, 32, device="cuda"), torch.randn(1, 2, 2, 2, 8, device="cuda")
+    one = (1, 1, 1)
+    with pytest.raises(RuntimeError, match=r"dont match: \(32 vs 24\)"):
+        DCNv4Function.apply(value, offset, one, one, (0, 0, 0), one, 3, 8, 1.0)

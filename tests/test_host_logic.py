@@ -85,6 +85,12 @@ def test_cpu_tensors_raise_instead_of_falling_back():
         FlashDeformAttnFunction.apply(value, shapes, lsi, packed, 1, 4, True)
 
 
+def test_binding_shares_the_process_libstdcxx():
+    """With a second, static copy inside the binding an error message that formats a number crashes instead of raising."""
+    with open(ops3d_b200._C.__file__, "rb") as f:
+        assert b"libstdc++.so.6\0" in f.read()
+
+
 def test_product_package_never_touches_the_oracle():
     """The oracle is test infrastructure: nothing under ops3d_b200/ (Python or C++/CUDA) may import,
     include, load or call it, and the package has no CPU code path to fall back to."""

@@ -154,6 +154,12 @@ at::Tensor flash_deform_attn(const at::Tensor &value, const at::Tensor &spatial_
         throw std::invalid_argument("sampling_loc_attn last dimension (" + std::to_string(last) +
                                     ") does not match value_spatial_shapes level count L=" + std::to_string(L) + " and K=" +
                                     std::to_string(K) + " (expected " + std::to_string(L * K * 4) + ")");
+    if (value.dim() == 4) {  // findspec_bwd's limit, which the kernels do not need: the operator refuses what it always refused
+        const int64_t G = value.size(2), C = value.size(3);
+        int64_t d_stride = 1;
+        while (d_stride < 32 && C % (2 * d_stride) == 0) d_stride *= 2;
+        TORCH_CHECK(G * (C / d_stride) <= 256, "Cannot fit G=", G, ", C=", C, " into 256 threads");
+    }
     at::Tensor output = flash_deform_attn_forward(value, spatial_shapes, level_start_index, sampling_loc_attn, im2col_step, K, 8, 0, use_reg);
     if (fda_nodes::needs_node({value, sampling_loc_attn})) {
         auto node = std::make_shared<FlashDeformAttnBackward>();

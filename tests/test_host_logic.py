@@ -91,6 +91,21 @@ def test_binding_shares_the_process_libstdcxx():
         assert b"libstdc++.so.6\0" in f.read()
 
 
+@pytest.mark.parametrize("heads,channels,fits", [(257, 8, False), (32, 8, True), (65, 12, True), (86, 12, False), (512, 32, False),
+                                                 (256, 32, True), (129, 64, False)])
+def test_more_heads_than_the_launch_hint_can_fit_are_refused(heads, channels, fits):
+    """``findspec_bwd`` raises where no channel stride fits 256 threads; the operator has always computed it."""
+    shapes, lsi = torch.tensor([[1, 1, 1]]), torch.tensor([0])
+    value, packed = torch.rand(1, 1, heads, channels), torch.rand(1, 1, heads, 16)
+    with pytest.raises(RuntimeError) as hint:
+        findspec_bwd(1, 1, heads, channels)
+        raise RuntimeError("fits")
+    assert (str(hint.value) == "fits") == fits
+    with pytest.raises(RuntimeError) as info:   # CPU tensors are refused later
+        FlashDeformAttnFunction.apply(value, shapes, lsi, packed, 1, 4, True)
+    assert ("Cannot fit" in str(info.value)) == (not fits)
+
+
 def test_product_package_never_touches_the_oracle():
     """The oracle is test infrastructure: nothing under ops3d_b200/ (Python or C++/CUDA) may import,
     include, load or call it, and the package has no CPU code path to fall back to."""

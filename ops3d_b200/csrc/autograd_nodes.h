@@ -50,6 +50,8 @@ inline bool needs_node(std::initializer_list<std::reference_wrapper<const at::Te
 struct SavedNode : public torch::autograd::Node {
     std::array<SavedVariable, 4> saved;
     void save(size_t i, const at::Tensor &t) { saved[i] = SavedVariable(t, /*is_output=*/false); }
+    // The output's gradient; where nothing has one for it (a later function returned None), zeros, as a Function gets them.
+    at::Tensor grad_output(const variable_list &grads) const { return grads[0].defined() ? grads[0] : input_metadata(0).zeros_like(); }
     at::Tensor unpack(size_t i) const { return saved[i].unpack(); }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);

@@ -139,10 +139,10 @@ struct FlashDeformAttnBackward : public fda_nodes::SavedNode {
     std::string name() const override { return "FlashDeformAttnFunctionBackward"; }
     torch::autograd::variable_list apply(torch::autograd::variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
-        if (!grads[0].defined()) return {at::Tensor(), at::Tensor()};
-        const bool recording = at::GradMode::is_enabled() && grads[0].requires_grad();
+        const at::Tensor grad = grad_output(grads);
+        const bool recording = at::GradMode::is_enabled() && grad.requires_grad();
         at::NoGradGuard no_grad;
-        auto r = flash_deform_attn_backward(unpack(0), unpack(1), unpack(2), unpack(3), grads[0].contiguous(), im2col_step, K, 1, 0);
+        auto r = flash_deform_attn_backward(unpack(0), unpack(1), unpack(2), unpack(3), grad.contiguous(), im2col_step, K, 1, 0);
         return fda_nodes::once_differentiable({r[0], r[1]}, recording);
     }
 };
@@ -263,12 +263,12 @@ struct DCNv4Backward : public fda_nodes::SavedNode {
     std::string name() const override { return "DCNv4FunctionBackward"; }
     torch::autograd::variable_list apply(torch::autograd::variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
-        if (!grads[0].defined()) return {at::Tensor(), at::Tensor()};
-        const bool recording = at::GradMode::is_enabled() && grads[0].requires_grad();
+        const at::Tensor grad = grad_output(grads);
+        const bool recording = at::GradMode::is_enabled() && grad.requires_grad();
         at::NoGradGuard no_grad;
         auto r = dcnv4_backward(unpack(0), unpack(1), a.kernel[0], a.kernel[1], a.kernel[2], a.stride[0], a.stride[1], a.stride[2],
                                 a.pad[0], a.pad[1], a.pad[2], a.dilation[0], a.dilation[1], a.dilation[2], a.group, a.group_channels,
-                                a.offset_scale, a.im2col_step, grads[0].contiguous(), a.remove_center, 8, 0, a.softmax);
+                                a.offset_scale, a.im2col_step, grad.contiguous(), a.remove_center, 8, 0, a.softmax);
         return fda_nodes::once_differentiable({r[0], r[1]}, recording);
     }
 };
@@ -337,9 +337,8 @@ struct RoIAlign3DBackward : public fda_nodes::SavedNode {
     std::string name() const override { return "RoIAlign3DFunctionBackward"; }
     torch::autograd::variable_list apply(torch::autograd::variable_list &&grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
-        if (!grads[0].defined()) return {at::Tensor()};
         at::NoGradGuard no_grad;
-        const at::Tensor &g = grads[0];
+        const at::Tensor g = grad_output(grads);
         c10::cuda::CUDAGuard guard(g.device());
         at::Tensor accum = empty_on(g, feature_size, at::kFloat);
         accum.zero_();

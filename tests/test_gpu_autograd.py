@@ -66,6 +66,24 @@ def test_saved_inputs_are_version_checked(make):
         out.sum().backward()
 
 
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, grad):
+        return None
+
+
+@pytest.mark.parametrize("make", [_attention, _dcnv4, _roi_align])
+def test_an_output_without_a_gradient_counts_as_zeros(make):
+    inputs, op = make()
+    leaves = [t.clone().requires_grad_(True) for t in inputs]
+    for got, leaf in zip(torch.autograd.grad(_NoGradient.apply(op(*leaves)).sum(), leaves), leaves):
+        assert got.shape == leaf.shape and not got.any()
+
+
 def test_an_error_message_with_numbers_raises():
     value, offset = torch.randn(1, 2, 2, 2, 32, device="cuda"), torch.randn(1, 2, 2, 2, 8, device="cuda")
     one = (1, 1, 1)

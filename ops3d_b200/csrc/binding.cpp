@@ -372,6 +372,7 @@ at::Tensor roi_align_3d(const at::Tensor &features, const at::Tensor &rois, int 
 
 at::Tensor nms_3d(const at::Tensor &dets, const at::Tensor &scores, const float threshold) {
     TORCH_CHECK(dets.is_cuda() && scores.is_cuda(), "nms_3d: boxes and scores must be CUDA tensors (no CPU implementation)");
+    TORCH_CHECK(dets.numel() == 0 || dets.device() == scores.device(), "nms_3d: boxes and scores must be on the same device");
     c10::cuda::CUDAGuard guard(dets.device());
     if (dets.numel() == 0) return at::empty({0}, dets.options().dtype(at::kLong));
     TORCH_CHECK(dets.dim() == 2 && dets.size(1) == 6, "boxes must be [N, 6] = (x1, y1, z1, x2, y2, z2)");

@@ -106,6 +106,16 @@ def test_more_heads_than_the_launch_hint_can_fit_are_refused(heads, channels, fi
     assert ("Cannot fit" in str(info.value)) == (not fits)
 
 
+def test_nms_refuses_scores_on_another_device():
+    """The ranking kernel reads both tensors by address.  Fake tensors: devices without memory, so nothing is launched here."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    with FakeTensorMode():
+        boxes, scores = torch.empty(4, 6, device="cuda:0"), torch.empty(4, device="cuda:1")
+        with pytest.raises(RuntimeError, match="same device"):
+            ops3d_b200._C.nms_3d(boxes, scores, 0.5)
+
+
 def test_product_package_never_touches_the_oracle():
     """The oracle is test infrastructure: nothing under ops3d_b200/ (Python or C++/CUDA) may import,
     include, load or call it, and the package has no CPU code path to fall back to."""

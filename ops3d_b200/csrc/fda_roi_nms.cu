@@ -5,9 +5,9 @@
 // (csrc/cuda/roi_align_3d_cuda_kernel.cuh:31,110) with their interpolation helpers
 // (csrc/cuda/interpolation_helpers_3d.h), and nms_kernel_3d plus the host-side greedy sweep of nms_3d_cuda
 // (csrc/cuda/nms_3d_cuda.cu:49-101,133-157).  Differences in structure, not in results:
-//   * ROI-Align: one thread per output element as in the reference, but the ROI geometry is computed once per
-//     thread in registers with the sample loops fully predicated; 16-bit features are read directly and
-//     accumulated in fp32;
+//   * ROI-Align: a warp per ROI and pair of channels contracts the volume axis after axis with one weight table per axis and
+//     ROI; one thread per output element as in the reference where the tables do not fit shared memory.  16-bit features are
+//     read directly and accumulated in fp32;
 //   * NMS: boxes are ranked by score, the pairwise-IoU bit matrix is built 64 x 64 boxes per block as in the reference,
 //     and the greedy sweep runs on the DEVICE in one block, so the matrix never crosses PCIe and the host only reads
 //     the number of kept boxes.
@@ -184,104 +184,174 @@ __global__ void __launch_bounds__(256) roi_align3d_backward_kernel(size_t total,
 // ---- separable form -------------------------------------------------------------------------------------
 // A sample's weights are products of one factor per axis, and so is its validity: the samples of a bin average to
 //   out[pd][ph][pw] = 1/count * sum_z Wz[pd][z] sum_y Wy[ph][y] sum_x Wx[pw][x] f[z][y][x]
-// with a small weight table per axis (nonzero on the bin's few voxels).  A block builds the tables of one ROI once for
+// over the voxels that samples touch, with a small weight table per axis.  A block builds the tables of one ROI once for
 // its channels; a warp takes one channel and contracts axis after axis, plane by plane: about 10 x fewer operations than
-// eight corners per sample, and in the backward one reduction per voxel of the ROI and channel instead of eight per
+// eight corners per sample, and in the backward one reduction per touched voxel of the ROI and channel instead of eight per
 // sample (7x7x7 bins of 2x2x2 samples on a 9x17x21 ROI: 3.2 k against 22 k).  256 ROIs x 128 channels of a 16x32x64 volume:
-// forward 652 -> 152 us, backward 1723 -> 166 us.  What bounds it: shared-memory and L1 accesses of the short dot products.
+// forward 648 -> 144 us, backward 1689 -> 160 us.  What bounds it: shared-memory and L1 accesses of the short dot products.
+//
+// The tables list the touched voxels only, in order.  A ROI with fewer samples than voxels leaves gaps between them; a voxel
+// in a gap is neither read nor added to, whatever it holds (its weight of zero would turn an infinity into NaN), and costs
+// nothing (64 ROIs over all of a 32x64x256 volume, 3x3x3 bins of 2x2x2 samples, 128 channels: by ranges of voxels forward 5.8
+// ms, backward 2.3; by lists 0.08 and 0.08).  A bin touches a contiguous part of an axis's list: bins and their samples lie in increasing order.
 struct AxisTable {
-    float *w;     // [bins][size], zero outside [lo, hi]
-    int *lo, *hi; // [bins] first / last voxel of a bin (hi < lo: no valid sample)
-    int *b0, *b1; // [size] first / last bin that reads a voxel (b1 < b0: none)
-    int bins, size;
+    float *w;     // [bins][size] weight of the i-th touched voxel, zero outside the bin's part
+    int *lo, *hi; // [bins] the bin's part of the list (hi < lo: no valid sample)
+    int *range;   // [size] first | last << 16 bin that touches the i-th touched voxel
+    int *vox;     // [size] the i-th touched voxel
+    int bins, size, n;
+    __device__ __forceinline__ int first_bin(int i) const { return range[i] & 0xffff; }
+    __device__ __forceinline__ int last_bin(int i) const { return (int)((unsigned int)range[i] >> 16); }
 };
 
 constexpr int kRoiThreads = 256;
 constexpr int kRoiChannels = 2;  // per warp at a time; 1 / 2 / 4: 484 / 317 / 399 us for the two passes below
 
 __host__ __device__ inline int roi_table_words(int bins, int size) { return bins * size + 2 * bins + 2 * size; }
+// All tables of a ROI: four words for the lengths of the lists, then x (its weights first, on a 16-byte boundary), y, z.
+__host__ __device__ inline int roi_tables_words(int pd, int ph, int pw, int depth, int height, int width) {
+    return 4 + roi_table_words(pd, depth) + roi_table_words(ph, height) + roi_table_words(pw, width);
+}
 
 __device__ __forceinline__ AxisTable axis_table(float *mem, int bins, int size) {
     AxisTable t;
     t.w = mem;
     t.lo = reinterpret_cast<int *>(mem + bins * size);
     t.hi = t.lo + bins;
-    t.b0 = t.hi + bins;
-    t.b1 = t.b0 + size;
+    t.range = t.hi + bins;
+    t.vox = t.range + size;
     t.bins = bins;
     t.size = size;
     return t;
 }
 
-// One thread per bin; samples of a bin lie in increasing order.  The rows of t.w are zero.
-__device__ __forceinline__ void fill_axis_bin(const AxisTable &t, int p, float start, float bin, int grid, int order) {
-    int lo = 0, hi = -1;
+// f(first voxel, second voxel, weight of the second, weight of the first) for the valid samples of bin p along an axis.
+template <typename F>
+__device__ __forceinline__ void for_axis_samples(int size, int p, float start, float bin, int grid, int order, F f) {
     for (int i = 0; i < grid; ++i) {
         const float v = start + p * bin + ((float)i + .5f) * bin / (float)grid;
-        if (v < -1.0f || v > (float)t.size) continue;
+        if (v < -1.0f || v > (float)size) continue;
         int i0, i1;
         float l, h;
-        axis_setup(v, t.size, i0, i1, l, h);
+        axis_setup(v, size, i0, i1, l, h);
         if (order == 0) {
             l = l > 0.5f ? 1.f : 0.f;
             h = 1.f - l;
         }
-        if (hi < lo) lo = i0;
-        hi = i1;
-        t.w[p * t.size + i0] += h;
-        t.w[p * t.size + i1] += l;
+        f(i0, i1, l, h);
     }
-    t.lo[p] = lo;
-    t.hi[p] = hi;
+}
+
+// Writes the indices in [0, size) that satisfy `wanted`, in order; returns their number.  By a whole warp.  wanted(i) may
+// read list[i]: that place is written only after it.
+template <typename F>
+__device__ __forceinline__ int list_indices(int size, int *list, F wanted) {
+    const int lane = threadIdx.x & 31;
+    int n = 0;
+    for (int base = 0; base < size; base += 32) {
+        const bool is = base + lane < size && wanted(base + lane);
+        const unsigned int mask = __ballot_sync(0xffffffffu, is);
+        if (is) list[n + __popc(mask & ((1u << lane) - 1u))] = base + lane;
+        n += __popc(mask);
+    }
+    return n;
 }
 
 struct RoiTables {
     AxisTable z, y, x;
-    int z0, z1, y0, y1, x0, x1;  // voxel range of the ROI (every bin's range lies inside)
+    float *end;
 };
 
-// Called by the whole block; ends with a barrier.
-template <typename RT>
+// Called by the whole block; ends with a barrier.  kVec = 0: the forward.  Otherwise the backward, which
+// visits rows in vectors of kVec voxels: along x, w and range are by voxel (last < first: not touched), and vox and n list the
+// vectors with a touched voxel.
+template <typename RT, int kVec>
 __device__ __forceinline__ RoiGeom build_roi_tables(RoiTables &t, float *mem, const RT *roi, float spatial_scale, int sampling_ratio,
                                                     int order, int depth, int height, int width, int pd, int ph, int pw) {
+    constexpr bool kForward = kVec == 0;
     const RoiGeom g = roi_geometry<RT>(roi, spatial_scale, sampling_ratio, pd, ph, pw);
-    t.x = axis_table(mem, pw, width);  // first: its rows are read as 16-byte vectors when the width is a multiple of four
-    t.y = axis_table(mem + roi_table_words(pw, width), ph, height);
-    t.z = axis_table(mem + roi_table_words(pw, width) + roi_table_words(ph, height), pd, depth);
-    const int tid = threadIdx.x, total = roi_table_words(pw, width) + roi_table_words(ph, height) + roi_table_words(pd, depth);
-    for (int i = tid; i < total; i += blockDim.x) mem[i] = 0.f;
+    int *counts = reinterpret_cast<int *>(mem);
+    t.x = axis_table(mem + 4, pw, width);
+    t.y = axis_table(reinterpret_cast<float *>(t.x.vox + width), ph, height);
+    t.z = axis_table(reinterpret_cast<float *>(t.y.vox + height), pd, depth);
+    t.end = reinterpret_cast<float *>(t.z.vox + depth);
+    const int tid = threadIdx.x, warp = tid >> 5, warps = blockDim.x >> 5;
+    for (int i = tid; mem + i < t.end; i += blockDim.x) mem[i] = 0.f;
     __syncthreads();
-    for (int i = tid; i < pd + ph + pw; i += blockDim.x) {
-        if (i < pd) fill_axis_bin(t.z, i, g.start_d, g.bin_d, g.grid_d, order);
-        else if (i < pd + ph) fill_axis_bin(t.y, i - pd, g.start_h, g.bin_h, g.grid_h, order);
-        else fill_axis_bin(t.x, i - pd - ph, g.start_w, g.bin_w, g.grid_w, order);
+    auto axis = [&](int a) {  // a copy: a reference chosen at run time would put the tables into local memory
+        AxisTable x = t.x;
+        if (a == 1) x = t.y;
+        if (a == 2) x = t.z;
+        return x;
+    };
+    auto for_bin_samples = [&](int i, auto f) {  // bin i of all axes' bins: x, then y, then z
+        if (i < pw) for_axis_samples(width, i, g.start_w, g.bin_w, g.grid_w, order, [&](int i0, int i1, float l, float h) { f(0, i, i0, i1, l, h); });
+        else if (i < pw + ph) for_axis_samples(height, i - pw, g.start_h, g.bin_h, g.grid_h, order, [&](int i0, int i1, float l, float h) { f(1, i - pw, i0, i1, l, h); });
+        else for_axis_samples(depth, i - pw - ph, g.start_d, g.bin_d, g.grid_d, order, [&](int i0, int i1, float l, float h) { f(2, i - pw - ph, i0, i1, l, h); });
+    };
+    // touched voxels, marked in vox
+    for (int i = tid; i < pw + ph + pd; i += blockDim.x)
+        for_bin_samples(i, [&](int a, int, int i0, int i1, float, float) {
+            int *mark = axis(a).vox;
+            mark[i0] = 1;
+            mark[i1] = 1;
+        });
+    __syncthreads();
+    // their lists, and in range every voxel's place in its list (-1: not touched)
+    for (int a = warp; a < 3; a += warps) {
+        const AxisTable x = axis(a);
+        for (int v = tid & 31; v < x.size; v += 32) x.range[v] = -1;
+        const int n = list_indices(x.size, x.vox, [&](int v) { return x.vox[v] != 0; });
+        __syncwarp();
+        for (int i = tid & 31; i < n; i += 32) x.range[x.vox[i]] = i;
+        if ((tid & 31) == 0) counts[a] = n;
     }
     __syncthreads();
-    for (int i = tid; i < depth + height + width; i += blockDim.x) {
-        const AxisTable &a = i < depth ? t.z : (i < depth + height ? t.y : t.x);
-        const int v = i < depth ? i : (i < depth + height ? i - depth : i - depth - height);
-        int first = 0, last = -1;
-        for (int p = 0; p < a.bins; ++p)
-            if (a.lo[p] <= v && v <= a.hi[p]) {
+    t.x.n = counts[0]; t.y.n = counts[1]; t.z.n = counts[2];
+    // weights and every bin's part of the list
+    for (int i = tid; i < pw + ph + pd; i += blockDim.x) {
+        const AxisTable x = axis(i < pw ? 0 : (i < pw + ph ? 1 : 2));
+        const int p = i < pw ? i : (i < pw + ph ? i - pw : i - pw - ph);
+        int lo = x.size, hi = -1;
+        for_bin_samples(i, [&](int a, int, int i0, int i1, float l, float h) {
+            const int j0 = x.range[i0], j1 = x.range[i1];
+            lo = min(lo, j0);
+            hi = max(hi, j1);
+            float *w = x.w + p * x.size;
+            w[!kForward && a == 0 ? i0 : j0] += h;
+            w[!kForward && a == 0 ? i1 : j1] += l;
+        });
+        x.lo[p] = lo;
+        x.hi[p] = hi;
+    }
+    __syncthreads();
+    // bins by voxel
+    auto set_bins = [](const AxisTable &x, int at, int i) {
+        int first = 1, last = 0;
+        for (int p = 0; p < x.bins; ++p)
+            if (x.lo[p] <= i && i <= x.hi[p]) {
                 if (last < first) first = p;
                 last = p;
             }
-        a.b0[v] = first;
-        a.b1[v] = last;
-    }
-    auto range = [](const AxisTable &a, int &v0, int &v1) {
-        v0 = a.size;
-        v1 = -1;
-        for (int p = 0; p < a.bins; ++p)
-            if (a.lo[p] <= a.hi[p]) {
-                v0 = min(v0, a.lo[p]);
-                v1 = max(v1, a.hi[p]);
-            }
+        x.range[at] = first | last << 16;
     };
-    range(t.z, t.z0, t.z1);
-    range(t.y, t.y0, t.y1);
-    range(t.x, t.x0, t.x1);
+    for (int i = tid; i < t.y.n; i += blockDim.x) set_bins(t.y, i, i);
+    for (int i = tid; i < t.z.n; i += blockDim.x) set_bins(t.z, i, i);
+    if constexpr (!kForward) {
+        for (int v = tid; v < width; v += blockDim.x) set_bins(t.x, v, t.x.range[v]);  // no bin has a place -1
+        __syncthreads();
+        if (warp == 0) {
+            const int n = list_indices(width / kVec, t.x.vox, [&](int i) {
+                bool any = false;
+#pragma unroll
+                for (int e = 0; e < kVec; ++e) any |= t.x.first_bin(i * kVec + e) <= t.x.last_bin(i * kVec + e);
+                return any;
+            });
+            if (tid == 0) counts[3] = n;
+        }
+    }
     __syncthreads();
+    if constexpr (!kForward) t.x.n = counts[3];
     return g;
 }
 
@@ -298,14 +368,14 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_forward_separable_ker
     extern __shared__ __align__(16) float roi_smem[];
     const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     RoiTables t;
-    const RoiGeom g = build_roi_tables<T>(t, roi_smem, rois + (size_t)n * 7, spatial_scale, sampling_ratio, order, depth, height, width, pd, ph, pw);
-    const int tables = roi_table_words(pd, depth) + roi_table_words(ph, height) + roi_table_words(pw, width);
+    const RoiGeom g = build_roi_tables<T, 0>(t, roi_smem, rois + (size_t)n * 7, spatial_scale, sampling_ratio, order, depth, height, width, pd, ph, pw);
     const int bins = pd * ph * pw, rows_size = height * pw;
-    float *rows = roi_smem + ((tables + 3) & ~3) + warp * kC * (rows_size + bins), *tile = rows + kC * rows_size;
+    float *rows = t.end + warp * kC * (rows_size + bins), *tile = rows + kC * rows_size;
     const int rows_per_step = 32 / pw, lane_row = lane / pw, p = lane - lane_row * pw;
     const bool used = lane_row < rows_per_step;
     const int xlo = used ? t.x.lo[p] : 0, xhi = used ? t.x.hi[p] : -1;
     const float *wx = t.x.w + (used ? p : 0) * width;
+    const bool gaps = t.x.n > 0 && t.x.vox[t.x.n - 1] - t.x.vox[0] != t.x.n - 1;
     const int c_end = min(channels, ((int)blockIdx.y + 1) * channels_per_block);
     const size_t volume = (size_t)depth * height * width;
     for (int c = blockIdx.y * channels_per_block + warp * kC; c < c_end; c += warps * kC) {
@@ -314,18 +384,30 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_forward_separable_ker
 #pragma unroll
         for (int k = 0; k < kC; ++k) of[k] = (size_t)min(k, c_end - 1 - c) * volume;
         for (int i = lane; i < kC * bins; i += 32) tile[i] = 0.f;
-        for (int z = t.z0; z <= t.z1; ++z) {
+        for (int z = 0; z < t.z.n; ++z) {
+            const T *plane = vol + (size_t)t.z.vox[z] * height * width;
             if (used)
-                for (int y = t.y0 + lane_row; y <= t.y1; y += rows_per_step) {
-                    const T *src = vol + ((size_t)z * height + y) * width;
+                for (int y = lane_row; y < t.y.n; y += rows_per_step) {
+                    const T *src = plane + (size_t)t.y.vox[y] * width;
                     float acc[kC];
 #pragma unroll
                     for (int k = 0; k < kC; ++k) acc[k] = 0.f;
+                    if (gaps) {
 #pragma unroll 2
-                    for (int x = xlo; x <= xhi; ++x) {
-                        const float w = wx[x];
+                        for (int x = xlo; x <= xhi; ++x) {
+                            const float w = wx[x];
+                            const T *at = src + t.x.vox[x];
 #pragma unroll
-                        for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, ldf<T>(src + of[k] + x), acc[k]);
+                            for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, ldf<T>(at + of[k]), acc[k]);
+                        }
+                    } else {
+                        const T *first = src + t.x.vox[0];
+#pragma unroll 2
+                        for (int x = xlo; x <= xhi; ++x) {
+                            const float w = wx[x];
+#pragma unroll
+                            for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, ldf<T>(first + of[k] + x), acc[k]);
+                        }
                     }
 #pragma unroll
                     for (int k = 0; k < kC; ++k) rows[k * rows_size + y * pw + p] = acc[k];
@@ -343,7 +425,7 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_forward_separable_ker
 #pragma unroll
                         for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, rows[k * rows_size + y * pw + p], acc[k]);
                     }
-                    for (int d = t.z.b0[z]; d <= t.z.b1[z]; ++d) {
+                    for (int d = t.z.first_bin(z), last = t.z.last_bin(z); d <= last; ++d) {
                         const float w = t.z.w[d * depth + z];
                         float *o = tile + (d * ph + q) * pw + p;
 #pragma unroll
@@ -359,8 +441,9 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_forward_separable_ker
     }
 }
 
-// The transpose, plane by plane: grad rows contracted along z, expanded along y, then along x into the voxels of the ROI's
-// plane, which are added to grad_features: kVec = 4 consecutive voxels per 16-byte reduction where the rows allow it.
+// The transpose, plane by plane: grad rows contracted along z, expanded along y, then along x into the touched voxels of
+// the plane, which are added to grad_features: kVec = 4 consecutive voxels per 16-byte reduction where the rows allow it
+// (untouched voxels of such a vector get zeros).
 template <typename T, int kVec>
 __global__ void __launch_bounds__(kRoiThreads) roi_align3d_backward_separable_kernel(const T *__restrict__ grad_out, const float *__restrict__ rois,
                                                                                     float spatial_scale, int sampling_ratio, int order,
@@ -371,29 +454,32 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_backward_separable_ke
     extern __shared__ __align__(16) float roi_smem[];
     const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     RoiTables t;
-    const RoiGeom g = build_roi_tables<float>(t, roi_smem, rois + (size_t)n * 7, spatial_scale, sampling_ratio, order, depth, height, width, pd, ph, pw);
-    const int tables = roi_table_words(pd, depth) + roi_table_words(ph, height) + roi_table_words(pw, width);
+    const RoiGeom g = build_roi_tables<float, kVec>(t, roi_smem, rois + (size_t)n * 7, spatial_scale, sampling_ratio, order, depth, height, width, pd, ph, pw);
     const int bins = pd * ph * pw, rows_size = height * pw, plane_size = ph * pw;
-    float *rows = roi_smem + ((tables + 3) & ~3) + warp * kC * (rows_size + bins + plane_size), *tile = rows + kC * rows_size,
-          *plane = tile + kC * bins;
+    float *rows = t.end + warp * kC * (rows_size + bins + plane_size), *tile = rows + kC * rows_size, *plane = tile + kC * bins;
     const int rows_per_step = 32 / pw, lane_row = lane / pw, p = lane - lane_row * pw;
     const bool used = lane_row < rows_per_step;
-    const int ny = t.y1 - t.y0 + 1, v0 = t.x0 / kVec, nv = t.x1 / kVec - v0 + 1;  // vectors per row of the ROI
+    const int ny = t.y.n, nv = t.x.n;
     const int c_end = min(channels, ((int)blockIdx.y + 1) * channels_per_block);
     const size_t volume = (size_t)depth * height * width;
-    if (t.z1 < t.z0 || ny <= 0 || t.x1 < t.x0) return;  // no valid sample (uniform over the block)
+    if (t.z.n == 0 || ny == 0 || nv == 0) return;  // no valid sample (uniform over the block)
     for (int c = blockIdx.y * channels_per_block + warp * kC; c < c_end; c += warps * kC) {
         float *vol = grad_features + ((size_t)g.batch * channels + c) * volume;
         const T *src = grad_out + ((size_t)n * channels + c) * (size_t)bins;
         const int valid = min(kC, c_end - c);
-        for (int i = lane; i < kC * bins; i += 32) tile[i] = i < valid * bins ? ldf<T>(src + i) / g.count : 0.f;
+        bool finite = true;
+        for (int i = lane; i < kC * bins; i += 32) {
+            tile[i] = i < valid * bins ? ldf<T>(src + i) / g.count : 0.f;
+            finite &= isfinite(tile[i]);
+        }
+        finite = __all_sync(0xffffffffu, finite);
         __syncwarp();
-        for (int z = t.z0; z <= t.z1; ++z) {
+        for (int z = 0; z < t.z.n; ++z) {
             for (int i = lane; i < plane_size; i += 32) {
                 float acc[kC];
 #pragma unroll
                 for (int k = 0; k < kC; ++k) acc[k] = 0.f;
-                for (int d = t.z.b0[z]; d <= t.z.b1[z]; ++d) {
+                for (int d = t.z.first_bin(z), last = t.z.last_bin(z); d <= last; ++d) {
                     const float w = t.z.w[d * depth + z];
 #pragma unroll
                     for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, tile[k * bins + d * plane_size + i], acc[k]);
@@ -403,11 +489,11 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_backward_separable_ke
             }
             __syncwarp();
             if (used)
-                for (int y = t.y0 + lane_row; y <= t.y1; y += rows_per_step) {
+                for (int y = lane_row; y < ny; y += rows_per_step) {
                     float acc[kC];
 #pragma unroll
                     for (int k = 0; k < kC; ++k) acc[k] = 0.f;
-                    for (int q = t.y.b0[y]; q <= t.y.b1[y]; ++q) {
+                    for (int q = t.y.first_bin(y), last = t.y.last_bin(y); q <= last; ++q) {
                         const float w = t.y.w[q * height + y];
 #pragma unroll
                         for (int k = 0; k < kC; ++k) acc[k] = fmaf(w, plane[k * plane_size + q * pw + p], acc[k]);
@@ -416,10 +502,11 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_backward_separable_ke
                     for (int k = 0; k < kC; ++k) rows[k * rows_size + y * pw + p] = acc[k];
                 }
             __syncwarp();
+            float *plane_dst = vol + (size_t)t.z.vox[z] * height * width;
             int r = lane / nv, v = lane - r * nv;            // row and vector of this lane, advanced without divisions
             const int step_r = 32 / nv, step_v = 32 - step_r * nv;
             while (r < ny) {
-                const int y = t.y0 + r, x = (v0 + v) * kVec;
+                const int x = t.x.vox[v] * kVec;
                 float acc[kC][kVec];
 #pragma unroll
                 for (int k = 0; k < kC; ++k)
@@ -427,28 +514,38 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_backward_separable_ke
                     for (int e = 0; e < kVec; ++e) acc[k][e] = 0.f;
                 int first = t.x.bins, last = -1;
 #pragma unroll
-                for (int e = 0; e < kVec; ++e)
-                    if (t.x.b0[x + e] <= t.x.b1[x + e]) {
-                        first = min(first, t.x.b0[x + e]);
-                        last = max(last, t.x.b1[x + e]);
-                    }
-                for (int b = first; b <= last; ++b) {
-                    const float *w = t.x.w + b * width + x;
-                    float we[kVec];
-                    if constexpr (kVec == 4) {
-                        const float4 w4 = *reinterpret_cast<const float4 *>(w);
-                        we[0] = w4.x; we[1] = w4.y; we[2] = w4.z; we[3] = w4.w;
-                    } else {
-                        we[0] = w[0];
-                    }
-#pragma unroll
-                    for (int k = 0; k < kC; ++k) {
-                        const float u = rows[k * rows_size + y * pw + b];
-#pragma unroll
-                        for (int e = 0; e < kVec; ++e) acc[k][e] = fmaf(we[e], u, acc[k][e]);
+                for (int e = 0; e < kVec; ++e) {
+                    const int lo = t.x.first_bin(x + e), hi = t.x.last_bin(x + e);
+                    if (lo <= hi) {
+                        first = min(first, lo);
+                        last = max(last, hi);
                     }
                 }
-                float *dst = vol + ((size_t)z * height + y) * width + x;
+                auto add_bins = [&](auto all_voxels) {
+                    for (int b = first; b <= last; ++b) {
+                        const float *w = t.x.w + b * width + x;
+                        float we[kVec];
+                        if constexpr (kVec == 4) {
+                            const float4 w4 = *reinterpret_cast<const float4 *>(w);
+                            we[0] = w4.x; we[1] = w4.y; we[2] = w4.z; we[3] = w4.w;
+                        } else {
+                            we[0] = w[0];
+                        }
+                        bool touched[kVec];
+#pragma unroll
+                        for (int e = 0; e < kVec; ++e) touched[e] = all_voxels.value || (t.x.first_bin(x + e) <= b && b <= t.x.last_bin(x + e));
+#pragma unroll
+                        for (int k = 0; k < kC; ++k) {
+                            const float u = rows[k * rows_size + r * pw + b];
+#pragma unroll
+                            for (int e = 0; e < kVec; ++e)
+                                if (touched[e]) acc[k][e] = fmaf(we[e], u, acc[k][e]);
+                        }
+                    }
+                };
+                if (finite) add_bins(std::true_type{});
+                else add_bins(std::false_type{});  // zero times infinity only where the bin touches the voxel
+                float *dst = plane_dst + (size_t)t.y.vox[r] * width + x;
 #pragma unroll
                 for (int k = 0; k < kC; ++k)
                     if (k < valid) {
@@ -479,10 +576,10 @@ struct RoiLaunch {
 };
 bool roi_launch(int num_rois, int channels, int depth, int height, int width, int pd, int ph, int pw, bool backward, RoiLaunch &l) {
     if (pw > 32 || (double)pd * depth + (double)ph * height + (double)pw * width > 40000.0 || (double)pd * ph * pw > 40000.0) return false;
-    const size_t tables = (size_t)roi_table_words(pd, depth) + roi_table_words(ph, height) + roi_table_words(pw, width);
+    const size_t tables = (size_t)roi_tables_words(pd, ph, pw, depth, height, width);
     const size_t per_warp = kRoiChannels * ((size_t)height * pw + (size_t)pd * ph * pw + (backward ? (size_t)ph * pw : 0));
     l.threads = kRoiThreads;
-    auto bytes = [&]() { return (((tables + 3) & ~(size_t)3) + (size_t)(l.threads / 32) * per_warp) * sizeof(float); };
+    auto bytes = [&]() { return (tables + (size_t)(l.threads / 32) * per_warp) * sizeof(float); };
     while (l.threads > 32 && bytes() > 56 * 1024) l.threads /= 2;  // four blocks of an SM
     l.smem = bytes();
     if (l.smem > 200 * 1024) return false;

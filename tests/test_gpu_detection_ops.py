@@ -149,3 +149,31 @@ def test_roi_align3d_row_shapes(size, width):
         want_g = oracle.roi_align3d_backward(gout.numpy(), rois.numpy(), tuple(feats.shape), 1.0, ratio, 1)
         assert np.abs(out.detach().cpu().numpy() - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
         assert np.abs(grad.cpu().numpy() - want_g).max() <= 1e-4 * max(1.0, np.abs(want_g).max())
+
+
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("width", [32, 33])    # 16-byte reductions or not
+@pytest.mark.parametrize("size,ratio", [((3, 3, 3), 2), ((2, 3, 1), 1), ((7, 7, 7), 2), ((2, 2, 2), 0)])   # gaps between samples, or none
+def test_roi_align3d_infinities_stay_where_samples_touch(size, ratio, width, order):
+    """Infinities and NaN in the features or the output gradient reach what the samples' eight corners reach and nothing else,
+    the corners of weight zero among them."""
+    N, C, D, H = 1, 5, 9, 17
+    gen = torch.Generator().manual_seed(width)
+    rois = torch.tensor([[0, 0.3, 0.2, 0.1, 31.4, 16.3, 8.2], [0, 3.1, 2.3, 1.4, 12.7, 9.9, 5.2], [0, 20.2, 1.1, 2.3, 23.1, 15.2, 7.7]])
+    bad = torch.tensor([float("inf"), float("-inf"), float("nan")])
+    feats = torch.randn(N, C, D, H, width, generator=gen)
+    hit = torch.rand(feats.shape, generator=gen) < 0.01
+    feats[hit] = bad[torch.randint(0, 3, (int(hit.sum()),), generator=gen)]
+    f = feats.cuda().requires_grad_(True)
+    out = ops3d.roi_align_3d(f, rois.cuda(), size, 1.0, ratio, order)
+    gout = torch.randn(out.shape, generator=gen)
+    hit = torch.rand(gout.shape, generator=gen) < 0.05
+    gout[hit] = bad[torch.randint(0, 3, (int(hit.sum()),), generator=gen)]
+    (grad,) = torch.autograd.grad(out, f, gout.cuda())
+    with np.errstate(invalid="ignore"):
+        want = oracle.roi_align3d_forward(feats.numpy(), rois.numpy(), size, 1.0, ratio, order)
+        want_g = oracle.roi_align3d_backward(gout.numpy(), rois.numpy(), tuple(feats.shape), 1.0, ratio, order)
+    for got, ref in ((out.detach().cpu().numpy(), want), (grad.cpu().numpy(), want_g)):
+        ok = np.isfinite(ref)
+        assert (np.isfinite(got) == ok).all() and ok.any() and not ok.all()
+        assert np.abs(got[ok] - ref[ok]).max() <= 1e-4 * max(1.0, np.abs(ref[ok]).max())

@@ -65,6 +65,7 @@ fda::Config read_config() {
     c.sorted = 1;
     c.sort_grid_x = 0;
     c.touched = 1;
+    c.roi_separable = 1;
     if (const char *e = std::getenv("FDA_L2_KEEP_FRACTION")) c.l2_keep_fraction = std::atof(e);
     if (c.l2_keep_fraction < 0) c.l2_keep_fraction = 0;
     if (const char *e = std::getenv("FDA_BINNING")) c.binning = std::atoi(e) != 0;
@@ -83,6 +84,7 @@ fda::Config read_config() {
     if (const char *e = std::getenv("FDA_SORT_GRID_X")) c.sort_grid_x = std::atoi(e);
     if (c.sort_grid_x < 0) c.sort_grid_x = 0;
     if (const char *e = std::getenv("FDA_BWD_TOUCHED")) c.touched = std::atoi(e);
+    if (const char *e = std::getenv("FDA_ROI_SEPARABLE")) c.roi_separable = std::atoi(e);
     return c;
 }
 

@@ -18,6 +18,7 @@ struct Config {
     int sorted;               // FDA_BWD_SORT          cell-sorted backward: 0 off, 1 for large, dense problems, 2 whenever the shape allows (1)
     int sort_grid_x;          // FDA_SORT_GRID_X       blocks per batch element walking the sorted list (0 = fill the SMs once)
     int touched;              // FDA_BWD_TOUCHED       fda_backward zero-fills / converts only the image rows the points touch: 0 never, 1 when they can touch at most 60 % of it, 2 always (1)
+    int roi_separable;        // FDA_ROI_SEPARABLE     ROI-Align axis by axis: 0 never, 1 unless the call is small, 2 whenever the shape allows (1)
 };
 
 const Config &config();

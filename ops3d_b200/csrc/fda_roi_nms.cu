@@ -188,12 +188,12 @@ __global__ void __launch_bounds__(256) roi_align3d_backward_kernel(size_t total,
 // its channels; a warp takes one channel and contracts axis after axis, plane by plane: about 10 x fewer operations than
 // eight corners per sample, and in the backward one reduction per touched voxel of the ROI and channel instead of eight per
 // sample (7x7x7 bins of 2x2x2 samples on a 9x17x21 ROI: 3.2 k against 22 k).  256 ROIs x 128 channels of a 16x32x64 volume:
-// forward 648 -> 144 us, backward 1689 -> 160 us.  What bounds it: shared-memory and L1 accesses of the short dot products.
+// forward 648 -> 143 us, backward 1689 -> 152 us.  What bounds it: shared-memory and L1 accesses of the short dot products.
 //
 // The tables list the touched voxels only, in order.  A ROI with fewer samples than voxels leaves gaps between them; a voxel
 // in a gap is neither read nor added to, whatever it holds (its weight of zero would turn an infinity into NaN), and costs
 // nothing (64 ROIs over all of a 32x64x256 volume, 3x3x3 bins of 2x2x2 samples, 128 channels: by ranges of voxels forward 5.8
-// ms, backward 2.3; by lists 0.08 and 0.08).  A bin touches a contiguous part of an axis's list: bins and their samples lie in increasing order.
+// ms, backward 2.3; by lists 0.07 and 0.08).  A bin touches a contiguous part of an axis's list: bins and their samples lie in increasing order.
 struct AxisTable {
     float *w;     // [bins][size] weight of the i-th touched voxel, zero outside the bin's part
     int *lo, *hi; // [bins] the bin's part of the list (hi < lo: no valid sample)
@@ -567,14 +567,32 @@ __global__ void __launch_bounds__(kRoiThreads) roi_align3d_backward_separable_ke
     }
 }
 
-// Launch shape of the separable kernels, or false: a row of bins wider than a warp, or tables and tiles beyond shared
-// memory even for one warp, take the element-wise kernels.
+// Whether a call is left to the element-wise kernels: at most 2x2x2 samples per bin and few corners in all.  They start their
+// loads at once and use a thread per output element, 5 to 20 us however large the ROIs are; the separable form first builds
+// its tables and then walks the planes of a ROI one after the other, 9 us and up.  More samples are a serial chain in a thread
+// (4x4x4: 40 us and up), and past these counts of corners the element-wise kernels are bound by them (0.9 ps a load, 2.4 ps a
+// reduction).  Measured on 8 and 256 ROIs x 16 and 128 channels of 3 to 100 % of volumes up to 32x64x256, us element-wise
+// against separable, 2x2x2 samples: forward 2.8 M corners 9-11 / 17-200, 8 M 13-38 / 12-250, 17 M 39-55 / 32-90, 22 M 27-100 /
+// 19-300, 33 M 36-84 / 15-80; backward 1.8 M 12-20 / 13-30, 2.8 M 17-26 / 19-190, 8 M 31-96 / 15-80.  With adaptive sampling the
+// host knows only the most samples a bin can have inside the volume.
+bool roi_elementwise_pays(int num_rois, int channels, int depth, int height, int width, int pd, int ph, int pw, int sampling_ratio,
+                          bool backward) {
+    auto along = [&](int size, int bins) { return sampling_ratio > 0 ? (double)sampling_ratio : (double)((size + bins - 1) / bins); };
+    const double samples = along(depth, pd) * along(height, ph) * along(width, pw);
+    return samples <= 8.0 && (double)num_rois * channels * pd * ph * pw * samples * 8.0 <= (backward ? 3e6 : 16e6);
+}
+
+// Launch shape of the separable kernels, or false: a call that the element-wise kernels do faster, a row of bins wider than a
+// warp, or tables and tiles beyond shared memory even for one warp.
 struct RoiLaunch {
     int threads, channels_per_block;
     size_t smem;
     dim3 grid;
 };
-bool roi_launch(int num_rois, int channels, int depth, int height, int width, int pd, int ph, int pw, bool backward, RoiLaunch &l) {
+bool roi_launch(int num_rois, int channels, int depth, int height, int width, int pd, int ph, int pw, int sampling_ratio, bool backward,
+                RoiLaunch &l) {
+    const int mode = fda::config().roi_separable;
+    if (mode <= 0 || (mode == 1 && roi_elementwise_pays(num_rois, channels, depth, height, width, pd, ph, pw, sampling_ratio, backward))) return false;
     if (pw > 32 || (double)pd * depth + (double)ph * height + (double)pw * width > 40000.0 || (double)pd * ph * pw > 40000.0) return false;
     const size_t tables = (size_t)roi_tables_words(pd, ph, pw, depth, height, width);
     const size_t per_warp = kRoiChannels * ((size_t)height * pw + (size_t)pd * ph * pw + (backward ? (size_t)ph * pw : 0));
@@ -851,7 +869,7 @@ extern "C" int fda_roi_align3d_forward(const void *features, const void *rois, v
     if (total == 0) return FDA_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RoiLaunch l;
-    if (roi_launch(num_rois, channels, depth, height, width, pooled_depth, pooled_height, pooled_width, false, l)) {
+    if (roi_launch(num_rois, channels, depth, height, width, pooled_depth, pooled_height, pooled_width, sampling_ratio, false, l)) {
         auto launch = [&](auto kernel, auto *typed) -> int {
             using T = std::remove_pointer_t<decltype(typed)>;
             const cudaError_t e = roi_opt_in(kernel, l.smem);
@@ -890,7 +908,7 @@ extern "C" int fda_roi_align3d_backward(const void *grad_output, const float *ro
     if (total == 0) return FDA_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RoiLaunch l;
-    if (roi_launch(num_rois, channels, depth, height, width, pooled_depth, pooled_height, pooled_width, true, l)) {
+    if (roi_launch(num_rois, channels, depth, height, width, pooled_depth, pooled_height, pooled_width, sampling_ratio, true, l)) {
         const bool vec = width % 4 == 0 && (reinterpret_cast<uintptr_t>(grad_features) & 15u) == 0;
         auto launch = [&](auto kernel, const auto *typed) -> int {
             const cudaError_t e = roi_opt_in(kernel, l.smem);

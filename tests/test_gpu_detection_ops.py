@@ -133,9 +133,11 @@ def test_nms3d_order_of_ties_and_far_columns(n):
     assert keep.tolist() == order.cpu()[ranked].tolist()
 
 
+@pytest.mark.parametrize("separable", ["1", "2"])                                  # by size (the smaller ones element by element), always
 @pytest.mark.parametrize("size", [(1, 1, 1), (2, 5, 7), (3, 2, 31), (2, 1, 33)])   # rows of bins: one, 4 of a warp, one lane idle, too wide
 @pytest.mark.parametrize("width", [8, 9, 40])                                      # 16-byte reductions or not; more than 32 vectors
-def test_roi_align3d_row_shapes(size, width):
+def test_roi_align3d_row_shapes(size, width, separable, fda_env):
+    fda_env(FDA_ROI_SEPARABLE=separable)
     N, C, D, H = 2, 9, 5, 6
     gen = torch.Generator().manual_seed(width)
     feats = torch.randn(N, C, D, H, width * (4 if width == 40 else 1), generator=gen)
@@ -151,12 +153,14 @@ def test_roi_align3d_row_shapes(size, width):
         assert np.abs(grad.cpu().numpy() - want_g).max() <= 1e-4 * max(1.0, np.abs(want_g).max())
 
 
+@pytest.mark.parametrize("separable", ["0", "2"])
 @pytest.mark.parametrize("order", [0, 1])
 @pytest.mark.parametrize("width", [32, 33])    # 16-byte reductions or not
 @pytest.mark.parametrize("size,ratio", [((3, 3, 3), 2), ((2, 3, 1), 1), ((7, 7, 7), 2), ((2, 2, 2), 0)])   # gaps between samples, or none
-def test_roi_align3d_infinities_stay_where_samples_touch(size, ratio, width, order):
+def test_roi_align3d_infinities_stay_where_samples_touch(size, ratio, width, order, separable, fda_env):
     """Infinities and NaN in the features or the output gradient reach what the samples' eight corners reach and nothing else,
     the corners of weight zero among them."""
+    fda_env(FDA_ROI_SEPARABLE=separable)
     N, C, D, H = 1, 5, 9, 17
     gen = torch.Generator().manual_seed(width)
     rois = torch.tensor([[0, 0.3, 0.2, 0.1, 31.4, 16.3, 8.2], [0, 3.1, 2.3, 1.4, 12.7, 9.9, 5.2], [0, 20.2, 1.1, 2.3, 23.1, 15.2, 7.7]])
@@ -177,3 +181,20 @@ def test_roi_align3d_infinities_stay_where_samples_touch(size, ratio, width, ord
         ok = np.isfinite(ref)
         assert (np.isfinite(got) == ok).all() and ok.any() and not ok.all()
         assert np.abs(got[ok] - ref[ok]).max() <= 1e-4 * max(1.0, np.abs(ref[ok]).max())
+
+
+def test_roi_align3d_small_and_large_calls_agree(fda_env):
+    """Calls on both sides of the size at which the separable form takes over (16 M corners forward, 3 M backward)."""
+    gen = torch.Generator().manual_seed(3)
+    C, n, volume = 16, 47, (6, 12, 20)
+    feats = torch.randn(1, C, *volume, generator=gen).cuda().requires_grad_(True)
+    rois = _rois(n, 1, *volume, seed=9).cuda()
+    for size in ((4, 4, 4), (6, 6, 6), (7, 7, 7)):   # 3.08, 10.4 and 16.5 M
+        gout = torch.randn(n, C, *size, generator=gen).cuda()
+        results = []
+        for mode in ("1", "0", "2"):
+            fda_env(FDA_ROI_SEPARABLE=mode)
+            out = ops3d.roi_align_3d(feats, rois, size, 1.0, 2, 1)
+            results.append((out.detach(), torch.autograd.grad(out, feats, gout)[0]))
+        for out, grad in results[1:]:
+            assert torch.allclose(out, results[0][0], atol=1e-5) and torch.allclose(grad, results[0][1], atol=1e-4)

@@ -50,7 +50,7 @@ def _run(cmd, verbose):
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    srcs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))]
+    srcs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h"))]
     srcs.append(os.path.join(ROOT, "include", "fda_b200.h"))
     if not force and _newer(LIB, srcs):
         return LIB

@@ -28,3 +28,45 @@ def test_walk_matches_oracle(shapes, Q, D, vdt, pdt, fda_env):
     for got, ref, dt in ((gv, ref_gv, vdt), (gp, ref_gp, pdt)):
         bound = ulp[dt] * ref.abs() + 2e-5 * ref.abs().max()
         assert ((got.float().cpu() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("vdt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [16, 32, 48, 64])
+@pytest.mark.parametrize("masked", [False, True])
+def test_small_weights_keep_their_bits(D, vdt, masked, fda_env):
+    """Cells reached only through soft-max probabilities down to 1e-14, alone or beside points of a probability near one
+    whose output gradient is zero: the fp32 image must agree with the plain kernel's, relative to every element.  Output
+    gradients are not negative, so nothing cancels; a cell sums at most a few hundred terms, in fp32 and in another order
+    (relative error below 100 * 2^-24 in either kernel: errors of a sum of positive terms grow far slower than its length)."""
+    shapes, Q, G, K = [(4, 8, 8)], 96, 2, 8
+    gen = torch.Generator().manual_seed(D)
+    N = 256
+    sh, lsi = torch.tensor(shapes).cuda(), torch.zeros(1, dtype=torch.long).cuda()
+    # voxel positions on a grid of 1/64: exact in fp32; the last point of a row, the strong one, sits left of x = 2 or anywhere
+    voxel = torch.randint(0, 64 * 3, (1, Q, G, K, 3), generator=gen) / 64.0
+    voxel[..., 0] += 3.5
+    voxel[..., -1, 0] = torch.randint(0, 64 * (7 if masked else 2), (1, Q, G), generator=gen) / 64.0
+    loc = (voxel + 0.5) / torch.tensor([8.0, 8.0, 4.0])
+    logits = -20.0 - torch.rand(1, Q, G, K, generator=gen) * 12.0
+    logits[..., -1] = 0.0
+    packed = torch.cat([loc.reshape(1, Q, G, 3 * K), logits], -1).cuda()
+    grad_out = torch.rand(1, Q, G, D, generator=gen) + 0.5
+    if masked:  # rows with a gradient have small weights only
+        packed[:, ::2, :, 4 * K - 1] = -33.0
+        packed[:, ::2, :, 3 * K] = 0.0      # the first point is the strong one now, out of the way
+        packed[:, ::2, :, 0:3] = torch.tensor([0.06, 0.06, 0.12]).cuda()
+        grad_out[:, 1::2] = 0.0
+    v = torch.randn(1, N, G, D, generator=gen).to("cuda", vdt)
+    go = grad_out.reshape(1, Q, G * D).to("cuda", vdt)
+    images = []
+    for mode in ("0", "2"):
+        fda_env(FDA_BWD_SORT=mode, FDA_BINNING="0")
+        assert (capi.backward_path(v, packed, K) >= 2) == (mode == "2")
+        scratch = torch.empty(max(256, capi.scratch_bytes(v, packed, K)), dtype=torch.uint8, device="cuda")
+        image, gp = torch.empty(v.shape, dtype=torch.float32, device="cuda"), torch.empty_like(packed)
+        capi.backward_accumulate_levels(v, sh, lsi, packed, go, K, image, gp, 0, 1, capi.BWD_ZERO_IMAGE | capi.BWD_FINALIZE, scratch=scratch)
+        images.append(image.double())
+    plain, got = images
+    reached = plain > 0
+    assert torch.equal(reached, got > 0) and plain[reached].min() < 1e-8
+    assert ((got - plain).abs() <= 200 * 2.0 ** -24 * plain).all()

@@ -35,6 +35,7 @@ constexpr int kScanItems = 8;                         // counters per thread of 
 constexpr int kScanThreads = 1024;
 constexpr int kScanTile = kScanItems * kScanThreads;  // counters per scan block
 constexpr unsigned int kNoPosition = 0xffffffffu;     // a point without a corner inside its level
+constexpr unsigned int kNotFinite = 0xfffffff0u;      // the same, and axes (bits x, y, z) whose position is not finite
 
 // Bins of one batch element: level l's start at first[l], head g's inside it at g * cells[l].  first[L] = all of them.
 // Bins of a coarse level lie stride[l] counters apart (the ones between stay empty): a level of 21 cells takes 5.7 M atomics
@@ -57,7 +58,8 @@ __device__ __forceinline__ void build_sort_bins(SortBins &s, const int64_t *shap
     s.first[L] = at;
 }
 
-// Base cell of a point from its normalised coordinates, and whether any corner lies inside the level.
+// Base cell of a point from its normalised coordinates, and whether any corner lies inside the level.  A NaN position is
+// cell 0, as in the plain kernel's conversion, with fractions of NaN.
 struct BaseCell {
     bool ok;
     int x, y, z;        // in [-1, size-1] when ok
@@ -67,11 +69,17 @@ __device__ __forceinline__ BaseCell base_cell(const LevelGeom &lv, float x, floa
     const float xv = unnormalize(x, lv.fW), yv = unnormalize(y, lv.fH), zv = unnormalize(z, lv.fD);
     const float xf = floorf(xv), yf = floorf(yv), zf = floorf(zv);
     BaseCell c;
-    // an axis has a corner in range iff floor in [-1, size-1]; written so that NaN fails
-    c.ok = (xf >= -1.f) && (xf <= lv.fW - 1.0f) && (yf >= -1.f) && (yf <= lv.fH - 1.0f) && (zf >= -1.f) && (zf <= lv.fD - 1.0f);
-    c.x = c.ok ? (int)xf : 0; c.y = c.ok ? (int)yf : 0; c.z = c.ok ? (int)zf : 0;
+    c.x = (int)xf; c.y = (int)yf; c.z = (int)zf;  // saturates
+    // an axis has a corner in range iff floor in [-1, size-1]
+    c.ok = (unsigned int)c.x + 1u <= (unsigned int)lv.W && (unsigned int)c.y + 1u <= (unsigned int)lv.H && (unsigned int)c.z + 1u <= (unsigned int)lv.D;
     c.fx = __fsub_rn(xv, xf); c.fy = __fsub_rn(yv, yf); c.fz = __fsub_rn(zv, zf);
     return c;
+}
+// Of a point that is not filed: infinite positions leave weights of infinity minus infinity times zero (the fraction is
+// NaN), which its gradients have to show.
+__device__ __forceinline__ unsigned int unfiled_code(const BaseCell &c) {
+    const unsigned int bad = (isfinite(c.fx) ? 0u : 1u) | (isfinite(c.fy) ? 0u : 2u) | (isfinite(c.fz) ? 0u : 4u);
+    return bad ? kNotFinite + bad : kNoPosition;
 }
 __device__ __forceinline__ unsigned int bin_of(const LevelGeom &lv, const BaseCell &c) {  // inside its level and head
     return ((unsigned int)(c.z + 1) * (unsigned int)(lv.H + 1) + (unsigned int)(c.y + 1)) * (unsigned int)(lv.W + 1) + (unsigned int)(c.x + 1);
@@ -91,7 +99,7 @@ __global__ void __launch_bounds__(256) fda_sort_clear_kernel(const Problem p) {
 
 // What the passes tell each other about a row lies where its gradient will: the first 4*L*K of the 8*L*K or more bytes of
 // its row of grad_sampling_loc_attn hold the rank of every point inside its bin, then its position in the list
-// (kNoPosition: not filed); the next eight its soft-max statistics {max, 1 / sum}.
+// (kNotFinite and above: not filed); the next eight its soft-max statistics {max, 1 / sum}.
 template <typename PT>
 __device__ __forceinline__ unsigned int *row_slots(const Problem &p, size_t rowg) {
     return reinterpret_cast<unsigned int *>(static_cast<PT *>(p.grad_packed) + rowg * (size_t)(4 * p.LK));
@@ -146,7 +154,8 @@ __global__ void __launch_bounds__(kThreads) fda_sort_count_kernel(const Problem 
                 const int l = (i >> 2) >> p.k_shift;
                 const LevelGeom lv = geom[l];
                 const BaseCell c = base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2]);
-                if (c.ok) rank[u] = atomicAdd(counters + bins.first[l] + g * bins.cells[l] + bin_of(lv, c) * bins.stride[l], 1u);
+                if (!c.ok) rank[u] = unfiled_code(c);
+                else rank[u] = atomicAdd(counters + bins.first[l] + g * bins.cells[l] + bin_of(lv, c) * bins.stride[l], 1u);
             }
         }
 #pragma unroll
@@ -211,7 +220,7 @@ __global__ void __launch_bounds__(kThreads) fda_sort_fill_kernel(const Problem p
             const int i = i0 + u * gs;
             pos[u] = i < LK ? ranks[i] : kNoPosition;
             start[u] = 0u;
-            if (pos[u] != kNoPosition) {
+            if (pos[u] < kNotFinite) {
                 const int l = (i >> 2) >> p.k_shift;
                 const LevelGeom lv = geom[l];
                 start[u] = __ldg(starts + bins.first[l] + g * bins.cells[l] +
@@ -221,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) fda_sort_fill_kernel(const Problem p
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
             const int i = i0 + u * gs;
-            if (pos[u] == kNoPosition) continue;
+            if (pos[u] >= kNotFinite) continue;
             const LevelGeom lv = geom[(i >> 2) >> p.k_shift];
             const BaseCell c = base_cell(lv, trow[3 * i], trow[3 * i + 1], trow[3 * i + 2]);
             const uint32_t sx = (uint32_t)p.GD, sy = (uint32_t)lv.W * sx, sz = (uint32_t)lv.H * sy;
@@ -747,7 +756,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 
 }
 
 // Per row: the results of its points from the list, soft-max backward grad_logit_i = p_i * (dalpha_i - sum_j p_j dalpha_j),
-// finished row of grad_sampling_loc_attn.  A point that is not filed has no result: its gradients are zero.  One random
+// finished row of grad_sampling_loc_attn.  A point that is not filed has no result: its gradients are zero
+// (NaN across the axes of an infinite position).  One random
 // 16-byte read per point; scattered 16-byte writes in the walk instead cost as much when the results fit L2 and three times
 // the DRAM traffic when they do not.
 template <typename PT>
@@ -788,7 +798,13 @@ __global__ void __launch_bounds__(kThreads) fda_sort_finalize_kernel(const Probl
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
             r[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (at[u] != kNoPosition) r[u] = __ldcs(p.sort_results + at[u]);
+            if (at[u] < kNotFinite) {
+                r[u] = __ldcs(p.sort_results + at[u]);
+            } else if (at[u] != kNoPosition) {  // zero times the NaN weights of the other axes
+                const unsigned int bad = at[u] - kNotFinite;
+                const float nan = __int_as_float(0x7fffffff);
+                r[u] = make_float4(bad & 6u ? nan : 0.f, bad & 5u ? nan : 0.f, bad & 3u ? nan : 0.f, nan);
+            }
         }
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {

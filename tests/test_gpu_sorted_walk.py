@@ -101,3 +101,26 @@ def test_no_further_from_64_bits_than_the_plain_kernel(D, vdt, fda_env):
         got = [image, gp[..., :48], gp[..., 48:]]
         errors.append([((a.cpu().double() - b).norm() / b.norm()).item() for a, b in zip(got, want)])
     assert all(sorted_ <= 1.05 * plain for plain, sorted_ in zip(*errors)), errors
+
+
+@pytest.mark.parametrize("vdt,pdt", [(torch.bfloat16, torch.float32), (torch.float16, torch.float16)])
+@pytest.mark.parametrize("D", [16, 32, 48])
+def test_positions_that_are_not_finite(D, vdt, pdt, fda_env):
+    """NaN and infinite coordinates give NaN gradients where the plain kernel gives them, and nowhere else."""
+    shapes, Q, K = [(4, 5, 6), (2, 3, 3)], 60, 4
+    value, sh, lsi, packed, grad_out = fda_oracle.make_inputs(shapes, 2, Q, 2, D, K, seed=D, lo=-0.2, hi=1.2)
+    nan, inf = float("nan"), float("inf")
+    for n, point in enumerate([(nan, 0.4, 0.4), (0.4, inf, 0.4), (0.4, 0.4, -inf), (nan, inf, 0.4), (7.0, nan, 0.4), (nan, nan, nan),
+                               (inf, -inf, nan), (6e4, 0.4, -6e4)]):
+        packed[n % 2, 7 * n, 1, 3 * n:3 * n + 3] = torch.tensor(point)
+    v, pk, go = value.to("cuda", vdt), packed.to("cuda", pdt), grad_out.to("cuda", vdt)
+    results = []
+    for mode in ("0", "2"):
+        fda_env(FDA_BWD_SORT=mode, FDA_BINNING="0")
+        results.append(capi.backward(v, sh.cuda(), lsi.cuda(), pk, go, K))
+    ulp = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 0.0}
+    for a, b, dt in zip(*results, (vdt, pdt)):
+        ok = torch.isfinite(a)
+        assert torch.equal(ok, torch.isfinite(b)) and not ok.all()
+        a, b = a.float()[ok], b.float()[ok]
+        assert ((a - b).abs() <= 2 * ulp[dt] * a.abs() + 2e-5 * a.abs().max()).all()   # as in test_walk_matches_oracle, on both sides

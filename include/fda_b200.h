@@ -51,7 +51,7 @@ typedef enum fda_status {
     FDA_ERR_BAD_HEAD_DIM = 5,     /* head_dim not a multiple of a 16-byte vector, or head row > 512 bytes */
     FDA_ERR_BAD_SHAPE = 6,        /* a non-positive dimension, or a tensor too large for the index width */
     FDA_ERR_IM2COL_STEP = 7,      /* batch % min(batch, im2col_step) != 0 */
-    FDA_ERR_WORKSPACE = 8,        /* workspace missing or smaller than fda_backward_workspace_bytes() */
+    FDA_ERR_WORKSPACE = 8,        /* workspace missing or smaller than the part a call cannot do without */
     FDA_ERR_MISALIGNED = 9,       /* a tensor base address is not 16-byte aligned */
     FDA_ERR_CUDA = 10,            /* a CUDA runtime call or the kernel launch failed; see fda_last_cuda_error() */
     FDA_ERR_TOO_LARGE_STATIC = 11 /* problem exceeds a compiled-in capacity */
@@ -89,7 +89,7 @@ int fda_forward(const void *value, const int64_t *spatial_shapes, const int64_t 
                 int im2col_step, int d_stride, int block_thread, int use_reg, void *stream);
 
 /*
- * Bytes of device workspace fda_backward needs for this problem: the fp32 accumulation image of
+ * Bytes of device workspace with which fda_backward takes its fastest path for this problem: the fp32 accumulation image of
  * grad_value for 16-bit values (batch*num_value*num_heads*head_dim*4, rounded up to 256; none for
  * an fp32 value, which accumulates in place) plus, when the slab-binned path applies,
  * fda_backward_scratch_bytes().
@@ -155,8 +155,10 @@ void fda_reload_config(void);
  * chunk loop and cast-back of flash_deform_attn_cuda_backward, csrc/cuda/flash_deform_attn_cuda.cu:125-178.
  *
  * The library zero-fills what it accumulates into (workspace, or grad_value for fp32); both
- * outputs are fully written.  workspace must be 256-byte aligned and at least
- * fda_backward_workspace_bytes() long; it may be NULL when that is 0.  When the gradient image
+ * outputs are fully written.  workspace must be 256-byte aligned.  It holds the image first (batch * num_value *
+ * num_heads * head_dim fp32 numbers rounded up to 256 bytes; none for fp32 values), which it has to fit, then the
+ * scratch of the faster paths: a call with less than fda_backward_workspace_bytes() takes the slab-binned path when
+ * fda_backward_scratch_bytes() fit behind the image, else the plain one.  It may be NULL for fp32 values.  When the gradient image
  * of one batch element does not fit L2, the largest level is processed slab by slab (its points
  * are first sorted into z-slabs in the workspace) so that its part of the image stays L2-resident.
  */

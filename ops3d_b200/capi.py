@@ -217,6 +217,27 @@ def _scatter_launches(value, packed, K, first=True, last=True) -> int:
     return 5 if path == 1 else 1
 
 
+def _first_workspace(device, *sizes):
+    """The first of ``sizes`` bytes (descending) that memory is left for; ``None`` when none is wanted.  The faster paths' lists
+    are optional: a call that fits memory without them must not fail for them."""
+    for n, need in enumerate(sizes):
+        if need == 0:
+            return None
+        try:
+            return torch.empty((need + 3) // 4, dtype=torch.float32, device=device)
+        except torch.cuda.OutOfMemoryError:
+            if n + 1 == len(sizes):
+                raise
+    return None
+
+
+def allocate_scratch(value, packed, K, device):
+    """Scratch for launches like these: ``scratch_bytes``, what the slab-binned path needs when memory is short, or ``None``."""
+    B, N, G, D = value.shape
+    binned = load().fda_backward_scratch_bytes(B, N, G, D, _levels(packed, K), packed.shape[1], K, DTYPE_CODE[packed.dtype])
+    return _first_workspace(device, scratch_bytes(value, packed, K), int(binned))
+
+
 def backward(value, shapes, lsi, packed, grad_out, K, im2col_step=64, grad_value=None, grad_packed=None,
              workspace=None):
     """``fda_backward`` on CUDA tensors; returns ``(grad_value, grad_packed)``."""
@@ -225,9 +246,11 @@ def backward(value, shapes, lsi, packed, grad_out, K, im2col_step=64, grad_value
         grad_value = torch.empty_like(value)
     if grad_packed is None:
         grad_packed = torch.empty_like(packed)
-    need = workspace_bytes(value, packed, K)
-    if need and workspace is None:
-        workspace = torch.empty((need + 3) // 4, dtype=torch.float32, device=value.device)
+    if workspace is None:
+        need = workspace_bytes(value, packed, K)
+        image = 0 if value.dtype == torch.float32 else (value.numel() * 4 + 255) // 256 * 256
+        scratch = int(load().fda_backward_scratch_bytes(B, N, G, D, L, Q, K, DTYPE_CODE[packed.dtype]))
+        workspace = _first_workspace(value.device, need, min(need, image + scratch), image)
     with torch.cuda.device(value.device):
         check(load().fda_backward(
             value.data_ptr(), shapes.data_ptr(), lsi.data_ptr(), packed.data_ptr(), grad_out.data_ptr(),
@@ -468,10 +491,12 @@ def dcnv4_backward(value, p_offset, grad_output, kernel, stride, pad, dilation, 
     need = int(load().fda_dcnv4_backward_scratch_bytes(B, Din, Hin, Win, group, group_channels, _triple(kernel), _triple(stride),
                                                        _triple(pad), _triple(dilation), int(remove_center), int(bool(softmax)),
                                                        DTYPE_CODE[value.dtype]))
-    ws = torch.empty((need + 3) // 4, dtype=torch.float32, device=value.device) if need else None
+    ws = _first_workspace(value.device, need, int(load().fda_dcnv4_backward_workspace_bytes(B, Din, Hin, Win, group, group_channels,
+                                                                                             DTYPE_CODE[value.dtype])))
+    ws_bytes = ws.numel() * ws.element_size() if ws is not None else 0
     with torch.cuda.device(value.device):
         check(load().fda_dcnv4_backward(value.data_ptr(), p_offset.data_ptr(), grad_output.data_ptr(), grad_value.data_ptr(),
-                                        grad_offset.data_ptr(), ws.data_ptr() if ws is not None else None, need, B, Din, Hin,
+                                        grad_offset.data_ptr(), ws.data_ptr() if ws is not None else None, ws_bytes, B, Din, Hin,
                                         Win, group, group_channels, _triple(kernel), _triple(stride), _triple(pad),
                                         _triple(dilation), float(offset_scale), int(remove_center), int(bool(softmax)),
                                         p_offset.shape[-1], DTYPE_CODE[value.dtype], im2col_step, _stream(value)))

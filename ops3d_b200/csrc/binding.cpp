@@ -18,6 +18,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -32,6 +33,20 @@ at::Tensor empty_on(const at::Tensor &like, at::IntArrayRef size, at::ScalarType
     return at::detail::empty_cuda(size, dtype, like.device(), std::nullopt);
 }
 at::Tensor empty_as(const at::Tensor &like) { return empty_on(like, like.sizes(), like.scalar_type()); }
+
+// The first of `bytes` (descending) that memory is left for; undefined when none is wanted.  The faster backward paths keep a
+// list of 48 bytes and more per sampling point; a call that fits memory without it must not fail for it.
+at::Tensor first_workspace(const at::Tensor &like, std::initializer_list<size_t> bytes) {
+    for (auto it = bytes.begin(); it != bytes.end(); ++it) {
+        if (*it == 0) break;
+        try {
+            return empty_on(like, {(int64_t)((*it + 3) / sizeof(float))}, at::kFloat);
+        } catch (const c10::OutOfMemoryError &) {
+            if (it + 1 == bytes.end()) throw;
+        }
+    }
+    return at::Tensor();
+}
 
 int dtype_code(const at::Tensor &t, const char *name) {
     switch (t.scalar_type()) {
@@ -118,13 +133,12 @@ std::vector<at::Tensor> flash_deform_attn_backward(const at::Tensor &value, cons
     if (d.Q == 0 || d.B == 0) return {at::zeros_like(value), at::zeros_like(sampling_loc_attn)};
     at::Tensor grad_value = empty_as(value);
     at::Tensor grad_packed = empty_as(sampling_loc_attn);
-    const size_t ws_bytes = fda_backward_workspace_bytes(d.B, d.N, d.G, d.D, d.L, d.Q, K, vdt, pdt);
-    at::Tensor workspace;
-    void *ws_ptr = nullptr;
-    if (ws_bytes > 0) {
-        workspace = empty_on(value, {(int64_t)((ws_bytes + 3) / sizeof(float))}, at::kFloat);
-        ws_ptr = workspace.data_ptr();
-    }
+    const size_t all = fda_backward_workspace_bytes(d.B, d.N, d.G, d.D, d.L, d.Q, K, vdt, pdt);
+    const size_t image = vdt == FDA_DTYPE_F32 ? 0 : ((size_t)value.numel() * sizeof(float) + 255) & ~(size_t)255;
+    const size_t binned = std::min(all, image + fda_backward_scratch_bytes(d.B, d.N, d.G, d.D, d.L, d.Q, K, pdt));
+    const at::Tensor workspace = first_workspace(value, {all, binned, image});
+    void *ws_ptr = workspace.defined() ? workspace.data_ptr() : nullptr;
+    const size_t ws_bytes = workspace.defined() ? workspace.nbytes() : 0;
     const int rc = fda_backward(value.data_ptr(), spatial_shapes.data_ptr<int64_t>(), level_start_index.data_ptr<int64_t>(),
                                 sampling_loc_attn.data_ptr(), grad_output.data_ptr(), grad_value.data_ptr(),
                                 grad_packed.data_ptr(), ws_ptr, ws_bytes, d.B, d.N, d.G, d.D, d.L, d.Q, K, vdt, pdt,
@@ -235,14 +249,12 @@ std::vector<at::Tensor> dcnv4_backward(const at::Tensor &value, const at::Tensor
     c10::cuda::CUDAGuard guard(value.device());
     at::Tensor grad_value = empty_as(value);
     at::Tensor grad_offset = empty_as(p_offset);
-    const size_t ws_bytes = fda_dcnv4_backward_scratch_bytes(d.B, d.Din, d.Hin, d.Win, group, group_channels, kernel, stride, pad,
-                                                             dilation, remove_center, softmax ? 1 : 0, vdt);
-    at::Tensor workspace;
-    void *ws_ptr = nullptr;
-    if (ws_bytes > 0) {
-        workspace = empty_on(value, {(int64_t)((ws_bytes + 3) / sizeof(float))}, at::kFloat);
-        ws_ptr = workspace.data_ptr();
-    }
+    const size_t all = fda_dcnv4_backward_scratch_bytes(d.B, d.Din, d.Hin, d.Win, group, group_channels, kernel, stride, pad, dilation,
+                                                        remove_center, softmax ? 1 : 0, vdt);
+    const size_t image = fda_dcnv4_backward_workspace_bytes(d.B, d.Din, d.Hin, d.Win, group, group_channels, vdt);
+    const at::Tensor workspace = first_workspace(value, {all, image});
+    void *ws_ptr = workspace.defined() ? workspace.data_ptr() : nullptr;
+    const size_t ws_bytes = workspace.defined() ? workspace.nbytes() : 0;
     raise_status(fda_dcnv4_backward(value.data_ptr(), p_offset.data_ptr(), grad_output.data_ptr(), grad_value.data_ptr(),
                                     grad_offset.data_ptr(), ws_ptr, ws_bytes, d.B, d.Din, d.Hin, d.Win, group, group_channels,
                                     kernel, stride, pad, dilation, offset_scale, remove_center, softmax ? 1 : 0, d.padded, vdt,

@@ -776,14 +776,14 @@ int fda_backward(const void *value, const int64_t *spatial_shapes, const int64_t
                  int im2col_step, int d_stride, int block_thread, void *stream) {
     (void)d_stride; (void)block_thread;
     if (!grad_value) return FDA_ERR_NULL_POINTER;
-    const size_t need = fda_backward_workspace_bytes(batch, num_value, num_heads, head_dim, num_levels, num_query, num_points,
-                                                     value_dtype, packed_dtype);
     const size_t n = (size_t)batch * num_value * num_heads * head_dim;
     const size_t image_bytes = value_dtype == FDA_DTYPE_F32 ? 0 : round256(n * sizeof(float));
     float *accum = static_cast<float *>(grad_value);
-    if (need > 0 && (!workspace || workspace_bytes < need)) return FDA_ERR_WORKSPACE;
+    if (image_bytes > 0 && (!workspace || workspace_bytes < image_bytes)) return FDA_ERR_WORKSPACE;
     if (image_bytes > 0) accum = static_cast<float *>(workspace);
-    void *scratch = need > image_bytes ? static_cast<char *>(workspace) + image_bytes : nullptr;
+    // what is left of the workspace decides which of the faster paths the scatter can take
+    const size_t scratch_bytes = workspace ? workspace_bytes - image_bytes : 0;
+    void *scratch = scratch_bytes > 0 ? static_cast<char *>(workspace) + image_bytes : nullptr;
     if (!aligned16(grad_value)) return FDA_ERR_MISALIGNED;
     const bool touched = image_bytes > 0 && fda_backward_touched_rows(batch, num_value, num_heads, head_dim, num_levels,
                                                                       num_query, num_points, value_dtype);
@@ -792,7 +792,7 @@ int fda_backward(const void *value, const int64_t *spatial_shapes, const int64_t
                                             num_query, num_points, value_dtype, packed_dtype, im2col_step, 0,
                                             num_levels > 0 ? num_levels : 1,
                                             (touched ? FDA_BWD_ZERO_TOUCHED : FDA_BWD_ZERO_IMAGE) | FDA_BWD_FINALIZE,
-                                            scratch, need - image_bytes, stream);
+                                            scratch, scratch_bytes, stream);
     if (rc != FDA_OK || image_bytes == 0) return rc;
     if (touched)
         return fda_cast_grad_value_touched(accum, grad_value, spatial_shapes, level_start_index, sampling_loc_attn, batch,

@@ -566,7 +566,8 @@ bool dcn_sorted_pays(int D, double points, double density) {
 
 // Scratch of the cell-sorted backward, behind the fp32 image: [shape] [where groups start] [counters] [scan tile sums]
 // [soft-max statistics] [ranks] [entries] [results], 52 bytes per point; total 0 when the path is not taken.  A call is sorted `elements` batch
-// elements at a time, as many as keep the list at 32 M points (at least one), which bounds the scratch.
+// elements at a time, as many as keep the list at 32 M points, and at least one: the scratch does not grow with the batch, but
+// follows an element that is larger than that.  Without memory for it a caller passes the image alone (plain path).
 struct DcnSortLayout {
     size_t shape, regions, counters, tile_sums, stats, ranks, entries, results, total;
     int elements;

@@ -74,8 +74,7 @@ class HostStreamedStep:
         self.go_c = [torch.empty(1, self.chunk, G * D, dtype=value_dtype, device=dev) for _ in range(S)]
         self.out_c = [torch.empty(1, self.chunk, G * D, dtype=value_dtype, device=dev) for _ in range(S)]
         self.gp_c = [torch.empty(1, self.chunk, G, last, dtype=packed_dtype, device=dev) for _ in range(S)]
-        nscr = capi.scratch_bytes(self.value_d[:1], self.packed_c[0], K)
-        self.scratch = [torch.empty(nscr, dtype=torch.uint8, device=dev) if nscr else None for _ in range(S)]
+        self.scratch = [capi.allocate_scratch(self.value_d[:1], self.packed_c[0], K, dev) for _ in range(S)]
         self.up = torch.cuda.Stream(device=dev)
         self.comp = torch.cuda.Stream(device=dev)
         self.down = torch.cuda.Stream(device=dev)

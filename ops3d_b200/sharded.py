@@ -303,8 +303,7 @@ class PeerReducer:
             if t[1] != -t[97]:
                 raise RuntimeError("PeerReducer.backward: ranks hold different numbers of batch elements; "
                                    "shard the inputs with partition() / shard_rows()")
-        self._scratch = ([torch.empty(nbytes, dtype=torch.uint8, device=self.device) for _ in range(self.nb)]
-                         if nbytes else None)
+        self._scratch = [capi.allocate_scratch(value[:1], packed[:1], K, self.device) for _ in range(self.nb)] if nbytes else None
         self._schedule, self._schedule_key = schedule, key
 
     # ---- exchange --------------------------------------------------------------------------------------------

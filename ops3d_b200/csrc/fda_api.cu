@@ -2,6 +2,7 @@
 // dispatch and kernel launches.  No torch types, no allocation, nothing but the CUDA runtime.
 #include "../../include/fda_b200.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -413,9 +414,10 @@ template <typename VT>
 int launch_walk(const fda::Problem &p, cudaStream_t st) {
     auto walk = p.D == 16 ? fda::fda_sorted_walk_kernel<VT, 1> : (p.D == 32 ? fda::fda_sorted_walk_kernel<VT, 2>
                 : (p.D == 48 ? fda::fda_sorted_walk_kernel<VT, 3> : fda::fda_sorted_walk_kernel<VT, 4>));
-    const size_t walk_smem = sizeof(fda::WalkShared);
+    const size_t walk_smem = fda::walk_smem_bytes(p.L * p.G);
     if (int rc = ensure_smem(reinterpret_cast<const void *>(walk), walk_smem)) return rc;
-    const int per_sm = p.D <= 32 ? 4 : (p.D == 48 ? 3 : 2);  // resident blocks, by registers
+    int per_sm = p.D <= 32 ? 4 : (p.D == 48 ? 3 : 2);  // resident blocks, by registers; with over a thousand regions by shared memory
+    per_sm = std::min(per_sm, (int)((size_t)226 * 1024 / (walk_smem + 2048)));
     int gx = g_config.sort_grid_x;
     if (gx <= 0) gx = (per_sm * sm_count() + p.B - 1) / p.B;
     walk<<<dim3((unsigned)gx, (unsigned)p.B, 1), fda::kWalkWarps * 32, walk_smem, st>>>(p);

@@ -414,7 +414,7 @@ template <int KS> struct RowWords {
 
 constexpr int kWalkSpan = 128;     // list entries a warp takes at a time
 constexpr int kWalkWarps = 4;
-constexpr int kWalkRegions = 160;  // most (level, head) regions of one launch
+constexpr int kWalkRegions = 16384;  // most (level, head) regions of one launch: their tables lie in shared memory
 struct WalkBuffer {                // per warp, double-buffered; padded so that a unit may be read past its end
     float4 geo[kWalkSpan + 8];     // fractions along x, y, z, probability
     uint4 tag[kWalkSpan + 8];      // row, (in a unit's first entry) end of the unit, base offset, corner mask
@@ -423,6 +423,8 @@ struct WalkShared {
     WalkBuffer buf[kWalkWarps][2];
     float4 dots[kWalkWarps][2][kWalkSpan];  // dot products of a point with corners 0-3 / 4-7
 };
+// followed by the first entry and span of every region, and the end
+inline size_t walk_smem_bytes(int regions) { return sizeof(WalkShared) + ((size_t)regions + 1) * sizeof(uint2); }
 
 // The list of a (level, head) region is cut into spans, one warp each; a span into runs of points with the same cell, runs
 // into units of at most eight points; a warp takes two units at a time (halves A and B, one cell each).  With the eight
@@ -452,33 +454,33 @@ __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 
     using Mma = WarpMma<VT>;
     constexpr int kQuarter = 4 * KS;     // channels of a lane's part of a row
     __shared__ LevelGeom geom[kMaxLevels];
-    __shared__ unsigned int region_entry[kWalkRegions + 1], region_span[kWalkRegions + 1];  // first entry / span of every region
     extern __shared__ __align__(16) unsigned char walk_smem[];
     WalkShared &sm = *reinterpret_cast<WalkShared *>(walk_smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = blockIdx.y;
     const int level_begin = __ffs(p.level_mask) - 1, level_end = 32 - __clz(p.level_mask);  // a contiguous range
     const int regions = (level_end - level_begin) * p.G;
+    uint2 *region_table = reinterpret_cast<uint2 *>(walk_smem + sizeof(WalkShared));  // {first entry, first span}
     if (tid == 0) build_level_table(geom, p.shapes, p.lsi, p.L, p.GD, p.value_elem_bytes, true, p.l2_keep_bytes);
-    for (int r = tid; r <= regions; r += blockDim.x) region_entry[r] = p.sort_regions[(size_t)b * (p.L * p.G + 1) + level_begin * p.G + r];
+    for (int r = tid; r <= regions; r += blockDim.x) region_table[r].x = p.sort_regions[(size_t)b * (p.L * p.G + 1) + level_begin * p.G + r];
     __syncthreads();
     if (warp == 0) {
         unsigned int carry = 0;
         for (int r0 = 0; r0 <= regions; r0 += 32) {  // uniform trip count
             const int r = r0 + lane;
-            const unsigned int n = r < regions ? (region_entry[r + 1] - region_entry[r] + kWalkSpan - 1) / kWalkSpan : 0u;
+            const unsigned int n = r < regions ? (region_table[r + 1].x - region_table[r].x + kWalkSpan - 1) / kWalkSpan : 0u;
             unsigned int inc = n;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const unsigned int t = __shfl_up_sync(0xffffffffu, inc, d);
                 if (lane >= d) inc += t;
             }
-            if (r <= regions) region_span[r] = carry + inc - n;
+            if (r <= regions) region_table[r].y = carry + inc - n;
             carry += __shfl_sync(0xffffffffu, inc, 31);
         }
     }
     __syncthreads();
-    const unsigned int spans = region_span[regions];
+    const unsigned int spans = region_table[regions].y;
     const int tig = lane & 3, grp = lane >> 2;
     const uint64_t pol_keep = l2_policy_evict_last(), pol_stream = l2_policy_evict_first();
     const VT *go_base = static_cast<const VT *>(p.grad_out) + tig * kQuarter;
@@ -497,8 +499,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 
 
     auto request_span = [&](unsigned int sp, int r, int which) {  // copies a span's records; commits one (possibly empty) group
         if (sp < spans) {
-            const unsigned int w0 = region_entry[r] + (sp - region_span[r]) * kWalkSpan;
-            const unsigned int left = region_entry[r + 1] - w0, wn = left < (unsigned int)kWalkSpan ? left : (unsigned int)kWalkSpan;
+            const unsigned int w0 = region_table[r].x + (sp - region_table[r].y) * kWalkSpan;
+            const unsigned int left = region_table[r + 1].x - w0, wn = left < (unsigned int)kWalkSpan ? left : (unsigned int)kWalkSpan;
             WalkBuffer &bf = sm.buf[warp][which];
             const float4 *src = p.sort_entries + 2 * (size_t)w0;
             void *dst = (lane & 1) ? static_cast<void *>(bf.tag) : static_cast<void *>(bf.geo);
@@ -510,16 +512,16 @@ __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 
     const unsigned int stride = gridDim.x * kWalkWarps;
     unsigned int sp = blockIdx.x * kWalkWarps + warp;
     int region = 0, which = 0;
-    while (region < regions && sp >= region_span[region + 1]) ++region;
+    while (region < regions && sp >= region_table[region + 1].y) ++region;
     request_span(sp, region, 0);
     for (; sp < spans; sp += stride, which ^= 1) {
         int next_region = region;
-        while (next_region < regions && sp + stride >= region_span[next_region + 1]) ++next_region;
+        while (next_region < regions && sp + stride >= region_table[next_region + 1].y) ++next_region;
         request_span(sp + stride, next_region, which ^ 1);
         cp_async_wait<1>();
         __syncwarp();
-        const unsigned int w0 = region_entry[region] + (sp - region_span[region]) * kWalkSpan;
-        const unsigned int left = region_entry[region + 1] - w0;
+        const unsigned int w0 = region_table[region].x + (sp - region_table[region].y) * kWalkSpan;
+        const unsigned int left = region_table[region + 1].x - w0;
         const int wn = (int)(left < (unsigned int)kWalkSpan ? left : (unsigned int)kWalkSpan);
         const float4 *geo = sm.buf[warp][which].geo;
         uint4 *tag = sm.buf[warp][which].tag;

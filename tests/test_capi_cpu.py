@@ -118,6 +118,8 @@ def test_cell_sorted_path_selection_and_scratch_size():
     assert lib.fda_forward_head_group(4608, G, D, 2, 4608, 4, 2) == G  # volume fits L2: plain row order
     # one rank of a head-split job at 8 GPUs: one batch element, 2 heads, every query -- as dense as the whole problem
     assert lib.fda_backward_path(1, N, 2, D, L, Q, K, 2) == 2
+    # heads do not decide the path: 192 (level, head) regions
+    assert lib.fda_backward_path(1, 37376, 64, 32, 3, 37376, 8, 2) == 2
 
 
 def test_sparse_image_handling_selection_and_validation(fda_env):

@@ -124,3 +124,19 @@ def test_positions_that_are_not_finite(D, vdt, pdt, fda_env):
         assert torch.equal(ok, torch.isfinite(b)) and not ok.all()
         a, b = a.float()[ok], b.float()[ok]
         assert ((a - b).abs() <= 2 * ulp[dt] * a.abs() + 2e-5 * a.abs().max()).all()   # as in test_walk_matches_oracle, on both sides
+
+
+@pytest.mark.parametrize("G,D,levels", [(64, 32, 3), (40, 16, 5), (401, 16, 3), (600, 32, 2)])
+def test_many_heads(G, D, levels, fda_env):
+    """More (level, head) regions than the usual few dozen: 192, 200, and over a thousand, whose tables leave less room for blocks."""
+    shapes = [(2, 3, 4), (2, 2, 2), (1, 2, 1), (1, 1, 2), (1, 1, 1)][:levels]
+    value, sh, lsi, packed, grad_out = fda_oracle.make_inputs(shapes, 2, 30, G, D, 4, seed=G, lo=-0.3, hi=1.3)
+    v, pk, go = value.to("cuda", torch.bfloat16), packed.cuda(), grad_out.to("cuda", torch.bfloat16)
+    results = []
+    for mode in ("0", "2"):
+        fda_env(FDA_BWD_SORT=mode, FDA_BINNING="0")
+        assert (capi.backward_path(v, pk, 4) >= 2) == (mode == "2")
+        results.append(capi.backward(v, sh.cuda(), lsi.cuda(), pk, go, 4))
+    for a, b, ulp in zip(*results, (2.0 ** -8, 0.0)):
+        a, b = a.float(), b.float()
+        assert ((a - b).abs() <= 2 * ulp * a.abs() + 2e-5 * a.abs().max()).all()   # as in test_walk_matches_oracle, on both sides

@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(kSweepThreads) nms3d_sweep_kernel(int n, int c
                                                                     const int *__restrict__ order, long long *__restrict__ keep,
                                                                     int *__restrict__ num_keep) {
     extern __shared__ unsigned long long kept_words[];            // [col_blocks] kept boxes of every decided chunk
-    int *kept_before = reinterpret_cast<int *>(kept_words + col_blocks);  // [col_blocks] boxes kept in earlier chunks
+    int *kept_before = reinterpret_cast<int *>(kept_words + col_blocks);  // [col_blocks / 2, up] boxes kept before every even chunk
     __shared__ unsigned long long removed_by_far[2][32];          // chunk c: what chunks 0..c-2 remove, by warp, slot c % 2
     __shared__ unsigned long long near_words[kSweepAhead][2 * kNmsBlock];  // chunk c: the words of chunk c-1, then of c itself
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, far_thread = (int)threadIdx.x - 32;
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(kSweepThreads) nms3d_sweep_kernel(int n, int c
             const unsigned long long kept = (unsigned long long)kept_hi << 32 | kept_lo;
             if (lane == 0) {
                 kept_words[cb] = kept;
-                kept_before[cb] = total;
+                if (!(cb & 1)) kept_before[cb >> 1] = total;
             }
             total += __popcll(kept);
         } else {
@@ -836,8 +836,10 @@ __global__ void __launch_bounds__(kSweepThreads) nms3d_sweep_kernel(int n, int c
     }
     for (int r = threadIdx.x; r < n; r += kSweepThreads) {
         const unsigned long long kept = kept_words[r >> 6];
-        if (kept >> (r & 63) & 1ull)
-            keep[kept_before[r >> 6] + __popcll(kept & ((1ull << (r & 63)) - 1ull))] = order ? order[r] : r;
+        if (kept >> (r & 63) & 1ull) {
+            const int before = kept_before[r >> 7] + ((r >> 6 & 1) ? __popcll(kept_words[(r >> 6) - 1]) : 0);
+            keep[before + __popcll(kept & ((1ull << (r & 63)) - 1ull))] = order ? order[r] : r;
+        }
     }
     if (threadIdx.x == 0) *num_keep = total;
 }
@@ -947,8 +949,8 @@ size_t nms_mask_bytes(int num_boxes) {
 int launch_nms(const float *boxes_sorted, const int *order, int num_boxes, float iou_threshold, unsigned long long *mask,
                long long *keep, int *num_keep, cudaStream_t st) {
     const int col_blocks = (num_boxes + kNmsBlock - 1) / kNmsBlock;
-    const size_t smem = (size_t)col_blocks * (sizeof(unsigned long long) + sizeof(int));
-    if (smem > 200 * 1024) return FDA_ERR_TOO_LARGE_STATIC;  // over a million boxes
+    const size_t smem = (size_t)col_blocks * sizeof(unsigned long long) + ((size_t)col_blocks + 1) / 2 * sizeof(int);
+    if (smem > 200 * 1024) return FDA_ERR_TOO_LARGE_STATIC;  // 1.31 M boxes; the matrix of 1.24 M fills the memory of the GPU
     nms3d_mask_kernel<<<dim3((unsigned)col_blocks, (unsigned)col_blocks), kNmsBlock, 0, st>>>(num_boxes, iou_threshold, boxes_sorted, mask);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return status_of(e);

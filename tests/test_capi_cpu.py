@@ -176,3 +176,20 @@ def test_bin_plan_is_a_pure_host_function():
     assert capi.bin_plan(shapes, (2, 598016, 8, 32), 598016, 8) == (0, 32, 1)
     assert capi.bin_plan(shapes.flip(0), (1, 598016, 8, 32), 1000, 4) == (2, 32, 1)   # largest level last
     assert capi.bin_plan(torch.tensor([(16, 32, 128), (8, 16, 64)]), (1, 73728, 8, 32), 73728, 4) is None  # 75 MB image fits
+
+
+def test_nms_size_limit():
+    """What bounds the number of boxes is the bit matrix in device memory (n^2 / 8 bytes, 1.24 M boxes in 192 GB), not the sweep's
+    tables in shared memory.  The status comes before any launch; without a device, the first size past that check fails on the
+    missing device instead, so there is nothing to run this against on a GPU box."""
+    import torch
+
+    if torch.cuda.is_available():
+        pytest.skip("would launch")
+    lib = capi.load()
+    p = ctypes.c_void_p(256)
+    n = 1_240_000
+    assert n * n // 8 > 192e9
+    call = lambda n: lib.fda_nms3d(p, n, 0.5, p, lib.fda_nms3d_workspace_bytes(n), p, p, None)  # noqa: E731
+    assert call(n) == 10                # CUDA error: no device
+    assert call(1_320_000) == 11        # too large

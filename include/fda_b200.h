@@ -201,7 +201,7 @@ int fda_cast_grad_value(const float *accum, void *grad_value, size_t num_element
  * slab-binned path for the largest level when it is part of the range, and keeps the logit
  * gradients handed from launch to launch in fp32 when the offsets are 16-bit (without it they pass
  * through grad_sampling_loc_attn and are rounded to 16 bits once more on the way); with at least
- * fda_backward_sorted_scratch_bytes() bytes (when that is not 0) the launches take the cell-sorted
+ * fda_backward_list_scratch_bytes() bytes (when that is not 0) the launches take the cell-sorted
  * path instead: the first launch of a sequence (no FDA_BWD_RESUME) sorts the points of all levels
  * into the scratch, every launch walks its levels' part of the list, the FDA_BWD_FINALIZE launch
  * writes grad_sampling_loc_attn (it holds nothing meaningful before).  Pass the same scratch to

@@ -243,7 +243,7 @@ size_t dalpha_plane_bytes(int B, int G, int L, int Q, int K, int pdt) {
     return round256((size_t)B * Q * G * L * K * sizeof(float));
 }
 
-// Cell-sorted backward: [where regions start] [spare] [entries, 32 bytes per point] [results, 16 bytes per point].  The
+// Cell-sorted backward: [where regions start, in a block of 4 bytes per cell and head and their scan tiles] [entries, 32 bytes per point] [results, 16 bytes per point].  The
 // counters of the bins and the scan's tile sums live where the results will (the part grows when a sparse problem's
 // counters need more).  Zero when the path is switched off or the problem does not qualify: 16-bit values with
 // 16, 32, 48 or 64 channels per head only (whole k-steps of the walk's matrix products); point ids and list positions are
@@ -471,7 +471,7 @@ int launch_sorted(fda::Problem p, cudaStream_t st) {
 // (fda_backward_touched.cuh) instead of the whole image.  Worst case (no two points share a row) the two point
 // passes write and read 8 rows of D floats per point; the dense passes move the image 2.5 times.  Taken when the
 // points can touch at most 60 % of the image.  The slab-binned scatter only adds to touched rows, like the plain
-// one; the cell-sorted path is for 10 and more points per cell and head and keeps the dense handling.
+// one; the cell-sorted path is taken at densities that reach most of the image and keeps the dense handling.
 bool touched_rows_choice(const Shape &s) {
     if (s.vdt == FDA_DTYPE_F32 || g_config.touched <= 0) return false;
     if (sort_layout(s.B, s.N, s.G, s.D, s.L, s.Q, s.K, s.vdt).total) return false;

@@ -100,13 +100,18 @@ def test_cell_sorted_path_selection_and_scratch_size():
     r256 = lambda n: (n + 255) // 256 * 256  # noqa: E731
     tiles = (bins + 8191) // 8192
     want = r256(bins * 4) + r256(tiles * 4) + r256(points * 32) + r256(points * 16)
-    assert lib.fda_backward_sorted_scratch_bytes(B, N, G, D, L, Q, K, 2) == want     # bf16: counters, scan, records, results
+    assert lib.fda_backward_sorted_scratch_bytes(B, N, G, D, L, Q, K, 2) == want     # bf16: front block, records, results
     assert lib.fda_backward_sorted_scratch_bytes(B, N, G, D, L, Q, K, 1) == want     # fp16 too
     assert lib.fda_backward_path(B, N, G, D, L, Q, K, 2) == 2
     assert lib.fda_backward_workspace_bytes(B, N, G, D, L, Q, K, 2, 0) == B * N * G * D * 4 + want
     assert lib.fda_backward_sorted_scratch_bytes(B, N, G, D, L, Q, K, 0) == 0        # fp32 values: not this path
     assert lib.fda_backward_path(B, N, G, D, L, Q, K, 0) == 1                        # ... but the image exceeds L2: brick-binned
-    assert lib.fda_backward_sorted_scratch_bytes(B, N, G, 64, L, Q, K, 2) == 0       # 64 channels per head: not this path
+    assert lib.fda_backward_sorted_scratch_bytes(B, N, G, 64, L, Q, K, 2) == 0       # speaks for 32 channels per head only ...
+    for width in (16, 48, 64):                                                       # ... the other widths of the path:
+        assert lib.fda_backward_list_scratch_bytes(B, N, G, width, L, Q, K, 2) == want
+        assert lib.fda_backward_path(B, N, G, width, L, Q, K, 2) == 3
+    assert lib.fda_backward_list_scratch_bytes(B, N, G, D, L, Q, K, 2) == want
+    assert lib.fda_backward_list_scratch_bytes(B, N, G, 40, L, Q, K, 2) == 0 and lib.fda_backward_path(B, N, G, 40, L, Q, K, 2) == 1
     assert lib.fda_backward_sorted_scratch_bytes(B, N, G, D, L, Q // 16, K, 2) == 0  # 1.5 points per cell and head: too sparse
     assert lib.fda_backward_path(B, N, G, D, L, Q // 16, K, 2) == 1
     assert lib.fda_backward_sorted_scratch_bytes(1, 288, 4, 32, 2, 288, 4, 2) == 0   # a few thousand points: too small

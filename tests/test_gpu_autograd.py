@@ -89,3 +89,37 @@ def test_an_error_message_with_numbers_raises():
     one = (1, 1, 1)
     with pytest.raises(RuntimeError, match=r"dont match: \(32 vs 24\)"):
         DCNv4Function.apply(value, offset, one, one, (0, 0, 0), one, 3, 8, 1.0)
+
+
+@pytest.mark.parametrize("make", [_attention, _dcnv4, _roi_align])
+def test_side_streams_and_threads(make):
+    """A node's backward runs on the stream of its forward, whichever thread asks for it."""
+    import threading
+
+    inputs, op = make()
+    plain = [t.clone().requires_grad_(True) for t in inputs]
+    out = op(*plain)
+    gout = torch.randn_like(out)
+    want = torch.autograd.grad(out, plain, gout)
+    torch.cuda.synchronize()
+    results = [None] * 4
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(2_000_000)   # what the side stream does is late
+            leaves = [(t * 1).requires_grad_(True) for t in inputs]
+            mine = op(*leaves)
+            grads = torch.autograd.grad(mine, leaves, gout * 1)
+            results[i] = [mine.detach().clone()] + [g.clone() for g in grads]
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(results))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for got in results:
+        assert torch.equal(got[0], out.detach())
+        for a, b in zip(got[1:], want):
+            assert torch.allclose(a, b, atol=1e-4 * b.abs().max().item())   # the order of fp32 sums

@@ -446,8 +446,8 @@ inline size_t walk_smem_bytes(int regions) { return sizeof(WalkShared) + ((size_
 // volume fits L2 (76 % of its wavefronts: one per 64-byte row, two per reduction), by random 64-byte reads of grad_output
 // from DRAM on the largest: 4.7 M points 490 -> 263 us, 229.6 M points 19.3 -> 9.7 ms.
 //
-// A unit of fewer than eight points repeats its last point with weight zero (an infinite grad_output row then gives NaN
-// where a scalar sum gives infinity; both mark the same elements).
+// A unit of fewer than eight points repeats its last point with weight zero.  An infinite grad_output row gives NaN where a
+// scalar sum may give infinity (a weight's terms may be zero or of either sign); both mark the same elements.
 template <typename VT, int KS>
 __global__ void __launch_bounds__(kWalkWarps * 32, KS <= 2 ? 4 : (KS == 3 ? 3 : 2)) fda_sorted_walk_kernel(const Problem p) {
     static_assert(Vec16<VT>::kCPL == 8, "16-bit value dtypes only");
